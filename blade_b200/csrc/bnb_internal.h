@@ -193,20 +193,35 @@ __device__ __forceinline__ void pdl_wait() {
 #endif
 }
 
+struct ClusterGrid {  // grid whose CTAs form clusters of `z` along z (1: none)
+  dim3 grid;
+  unsigned z;
+};
+
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+inline cudaError_t launch_pdl(void (*kernel)(P...), ClusterGrid g, dim3 block, size_t smem, cudaStream_t s,
                               A &&...args) {
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = g.z;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
+  cfg.gridDim = g.grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = g.z > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                              A &&...args) {
+  return launch_pdl(kernel, ClusterGrid{grid, 1}, block, smem, s, std::forward<A>(args)...);
 }
 
 }  // namespace bnb

@@ -12,11 +12,20 @@
 // in FP32 in a fixed order on the tensor pipe (mma.sync m16n8k16), so results
 // are reproducible run to run.  act is
 // 0 (identity) or 1 (SiLU, z * sigmoid(z)).
+// All kernels are launched with programmatic dependent launch: at these sizes
+// a launch's latency is as long as its work.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "bnb.h"
+#include "bnb_internal.h"
+
+namespace cg = cooperative_groups;
+using bnb::ClusterGrid;
+using bnb::launch_pdl;
+using bnb::pdl_wait;
 
 namespace {
 
@@ -26,167 +35,381 @@ __device__ __forceinline__ uint16_t f2bf(float f) {
 }
 __device__ __forceinline__ float sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
 
-// C[i,j] = sum_l A(i,l) B(l,j) over BF16 operands given by strides:
-// A(i,l) = A[i*sai + l*sal], B(l,j) = B[l*sbl + j*sbj]; C row-major [I,J].
-// On the tensor pipe: a 64x64 output tile per 256-thread CTA, K staged in
-// 64s through shared memory (A as [row][k], B as [column][k]), each of the
-// 8 warps (2 x 4) computing 32x16 of the tile as 2 x 2 mma.m16n8k16 with
-// BF16 operands and FP32 accumulators, k steps of 16 in increasing order.
-constexpr int kT = 64, kK = 64, kPad = 8;
+// ---------------------------------------------------------------------------
+// Products C[i,j] = sum_l A(i,l) B(l,j) over dense BF16 operands.
+//
+// Each operand is stored with either the sum index l contiguous (A row-major
+// [I,L], B as [J,L]) or its own index contiguous (A as [L,I], B as [L,J]); it
+// is staged in shared memory as it is stored, and ldmatrix (.trans for the
+// second form) makes the fragments, so the forward product and both backward
+// products run through one kernel without a transposition.
+//
+// What bounds it: the network's products (256 x 256 x 1664 and smaller) hold
+// 0.01-0.2 GFLOP each, so a product lasts as long as the memory latencies one
+// CTA sees in a row.  Hence: T x T output tiles with T = 32 unless 64 still
+// gives half the SMs a tile, l in chunks of 64 through a ring of cp.async
+// buffers (7 chunks in flight at T = 32), and two products that do not depend
+// on one another (dW and dX) in one launch.  l is not split over CTAs: each
+// element is one chain of k16 steps in increasing order, so every result,
+// and with it every BF16 rounding downstream, is that of any other tiling.
+// Measured (B200, network 1664-256-256-256-128): a training step of batch 256
+// 487 -> 102 us, a forward pass of a small batch 215 -> 32 us against 64 x 64
+// tiles staged element by element without overlap (11 products of 52 us each),
+// separate bias/activation, column-sum and per-tensor Adam launches.
+// ---------------------------------------------------------------------------
+constexpr int kC = 64;       // l per chunk
 
-__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+struct Product {
+  const uint16_t *A, *B;
+  int I, J, L;
+  int lastA, lastB;   // 1: the operand's own index is contiguous (A as [L,I], B as [L,J])
+  int tilesJ, tiles;  // T x T output tiles
+  float *C;           // [I,J]
+  const float *bias;  // [J] or null
+  int act;            // forward only (Y or Yf set): 0 identity, 1 SiLU
+  uint16_t *Y;        // [I,J] BF16 of act(C + bias), or null
+  float *Yf;          // the same in FP32, or null
+};
+struct Products {
+  Product p[2];
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void *p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool in) {
+  const int n = in ? 16 : 0;  // 0 source bytes: the 16 are zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n));
+}
+__device__ __forceinline__ void ldsm4(uint32_t addr, bool trans, uint32_t (&r)[4]) {
+  if (trans)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-__global__ void __launch_bounds__(256) k_gemm_bf16(int I, int J, int Lk, const uint16_t *A, long long sai,
-                                                   long long sal, const uint16_t *B, long long sbl,
-                                                   long long sbj, float *C) {
-  __shared__ __align__(16) uint16_t sA[kT][kK + kPad];  // [tile row][k]
-  __shared__ __align__(16) uint16_t sB[kT][kK + kPad];  // [tile column][k]
-  const int i0 = blockIdx.y * kT, j0 = blockIdx.x * kT;
+// Shared-memory pitch (elements) of a staged operand: [T][kC] or [kC][T].  Both
+// pitches are odd multiples of 16 bytes, so the 8 rows of an ldmatrix matrix
+// fall into different banks.
+template <int T>
+__device__ __forceinline__ int pitch_of(bool last) {
+  return last ? T + 8 : kC + 8;
+}
+template <int T>
+constexpr int stages() {  // ring of chunks: 80 KB (T = 32) or 72 KB (T = 64) of shared memory
+  return T == 32 ? 8 : 4;
+}
+template <int T>
+constexpr int stage_elems() {
+  return T * (kC + 8) > kC * (T + 8) ? T * (kC + 8) : kC * (T + 8);
+}
+
+// Stages rows r0.. (own index) x l0.. of one operand; `last` as in Product.
+// VEC: 16-byte asynchronous copies (the contiguous extent is a multiple of 8
+// elements and the base 16-byte aligned, so a copy lies inside or outside as a
+// whole); otherwise element by element.
+template <int T, int THREADS, bool VEC>
+__device__ __forceinline__ void stage(uint16_t *dst, const uint16_t *src, int R, int L, bool last, int r0, int l0) {
+  const int pitch = pitch_of<T>(last);
+  if (VEC) {
+    const int cpr = last ? T / 8 : kC / 8;  // copies per staged row
+#pragma unroll
+    for (int c = threadIdx.x; c < T * kC / 8; c += THREADS) {
+      const int row = c / cpr, col = (c - row * cpr) * 8;
+      const int r = r0 + (last ? col : row), l = l0 + (last ? row : col);
+      const bool in = r < R && l < L;
+      const size_t at = last ? (size_t)l * R + r : (size_t)r * L + l;
+      cp_async16(smem_u32(dst + row * pitch + col), in ? src + at : src, in);
+    }
+  } else {
+    const int w = last ? T : kC;
+    for (int c = threadIdx.x; c < T * kC; c += THREADS) {
+      const int row = c / w, col = c - row * w;
+      const int r = r0 + (last ? col : row), l = l0 + (last ? row : col);
+      const size_t at = last ? (size_t)l * R + r : (size_t)r * L + l;
+      dst[row * pitch + col] = r < R && l < L ? src[at] : (uint16_t)0;
+    }
+  }
+}
+
+// T = 64: 2 x 4 warps of 32 x 16; T = 32: 2 x 2 warps of 16 x 16.
+template <int T, bool VEC>
+__global__ void __launch_bounds__(T == 64 ? 256 : 128) k_gemm_bf16(Products ps) {
+  pdl_wait();
+  constexpr int THREADS = T == 64 ? 256 : 128;
+  constexpr int WN = T / 16;      // warps along j
+  constexpr int MT = T / 32;      // 16-row fragments per warp (2 warps along i)
+  constexpr int STAGE = stage_elems<T>(), kStages = stages<T>();
+  extern __shared__ __align__(16) uint16_t sm[];
+  const Product &p = blockIdx.x < ps.p[0].tiles ? ps.p[0] : ps.p[1];
+  const int tile = blockIdx.x < ps.p[0].tiles ? blockIdx.x : blockIdx.x - ps.p[0].tiles;
+  const int i0 = tile / p.tilesJ * T, j0 = tile % p.tilesJ * T;
+  const bool tA = p.lastA != 0, tB = p.lastB != 0;
+  const int pA = pitch_of<T>(tA), pB = pitch_of<T>(tB);
+  const int n = (p.L + kC - 1) / kC;  // chunks of l
+
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wm = warp >> 2, wn = warp & 3;  // warp tile: rows wm*32.., columns wn*16..
-  const int g = lane >> 2, t = lane & 3;    // mma fragment coordinates
-  float acc[2][2][4] = {};
-  for (int l0 = 0; l0 < Lk; l0 += kK) {
-    for (int e = threadIdx.x; e < kK * kT; e += 256) {
-      const int r = e / kK, l = e % kK;  // r: tile row (A) or column (B), l: k index
-      const int gi = i0 + r, gj = j0 + r, gl = l0 + l;
-      sA[r][l] = (gi < I && gl < Lk) ? A[gi * sai + gl * sal] : (uint16_t)0;
-      sB[r][l] = (gj < J && gl < Lk) ? B[gl * sbl + gj * sbj] : (uint16_t)0;
+  const int wm = warp / WN * (MT * 16), wn = warp % WN * 16;  // warp's corner in the tile
+  const int mat = lane >> 3, r8 = lane & 7;
+  // element offsets of this lane's ldmatrix rows inside a stage, at k = 0
+  const int aoff = tA ? ((mat >> 1) * 8 + r8) * pA + wm + (mat & 1) * 8 : (wm + (mat & 1) * 8 + r8) * pA + (mat >> 1) * 8;
+  const int astep = tA ? 16 * pA : 16, arow = tA ? 16 : 16 * pA;
+  const int boff = tB ? ((mat & 1) * 8 + r8) * pB + wn + (mat >> 1) * 8 : (wn + (mat >> 1) * 8 + r8) * pB + (mat & 1) * 8;
+  const int bstep = tB ? 16 * pB : 16;
+
+  float acc[MT][2][4] = {};
+  auto load = [&](int c) {
+    if (c < n) {
+      uint16_t *s = sm + (c % kStages) * 2 * STAGE;
+      stage<T, THREADS, VEC>(s, p.A, p.I, p.L, tA, i0, c * kC);
+      stage<T, THREADS, VEC>(s + STAGE, p.B, p.J, p.L, tB, j0, c * kC);
     }
-    __syncthreads();
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
 #pragma unroll
-    for (int ks = 0; ks < kK; ks += 16) {
-      uint32_t af[2][4], bfr[2][2];
+  for (int c = 0; c < kStages - 1; c++) load(c);
+  for (int c = 0; c < n; c++) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 2) : "memory");
+    __syncthreads();  // chunk c is staged, and every warp is done with the buffer refilled next
+    load(c + kStages - 1);
+    const uint16_t *s = sm + (c % kStages) * 2 * STAGE;
+    const uint32_t aA = smem_u32(s + aoff), aB = smem_u32(s + STAGE + boff);
 #pragma unroll
-      for (int mt = 0; mt < 2; mt++) {
-        const int rb = wm * 32 + mt * 16;
-        af[mt][0] = *reinterpret_cast<const uint32_t *>(&sA[rb + g][ks + 2 * t]);
-        af[mt][1] = *reinterpret_cast<const uint32_t *>(&sA[rb + g + 8][ks + 2 * t]);
-        af[mt][2] = *reinterpret_cast<const uint32_t *>(&sA[rb + g][ks + 2 * t + 8]);
-        af[mt][3] = *reinterpret_cast<const uint32_t *>(&sA[rb + g + 8][ks + 2 * t + 8]);
+    for (int k = 0; k < kC / 16; k++) {
+      uint32_t a[MT][4], b[4];
+#pragma unroll
+      for (int m = 0; m < MT; m++) ldsm4(aA + 2 * (k * astep + m * arow), tA, a[m]);
+      ldsm4(aB + 2 * k * bstep, tB, b);
+#pragma unroll
+      for (int m = 0; m < MT; m++) {
+        mma_bf16_16816(acc[m][0], a[m], b[0], b[1]);
+        mma_bf16_16816(acc[m][1], a[m], b[2], b[3]);
       }
-#pragma unroll
-      for (int nt = 0; nt < 2; nt++) {
-        const int cb = wn * 16 + nt * 8;
-        bfr[nt][0] = *reinterpret_cast<const uint32_t *>(&sB[cb + g][ks + 2 * t]);
-        bfr[nt][1] = *reinterpret_cast<const uint32_t *>(&sB[cb + g][ks + 2 * t + 8]);
-      }
-#pragma unroll
-      for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-        for (int nt = 0; nt < 2; nt++) mma_bf16_16816(acc[mt][nt], af[mt], bfr[nt]);
     }
-    __syncthreads();
   }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  // the tile through shared memory, for whole-row stores
+  constexpr int PT = T + 4;
+  float *part = reinterpret_cast<float *>(sm);
 #pragma unroll
-  for (int mt = 0; mt < 2; mt++)
+  for (int m = 0; m < MT; m++)
 #pragma unroll
-    for (int nt = 0; nt < 2; nt++) {
-      const int row = i0 + wm * 32 + mt * 16 + g, col = j0 + wn * 16 + nt * 8 + 2 * t;
+    for (int q = 0; q < 2; q++)
 #pragma unroll
-      for (int h = 0; h < 2; h++) {  // h = 0: row g, h = 1: row g + 8
-        const int r = row + 8 * h;
-        if (r < I && col < J) C[(size_t)r * J + col] = acc[mt][nt][2 * h];
-        if (r < I && col + 1 < J) C[(size_t)r * J + col + 1] = acc[mt][nt][2 * h + 1];
+      for (int h = 0; h < 2; h++)
+        *reinterpret_cast<float2 *>(&part[(wm + 16 * m + 8 * h + (lane >> 2)) * PT + wn + 8 * q + 2 * (lane & 3)]) =
+            make_float2(acc[m][q][2 * h], acc[m][q][2 * h + 1]);
+  __syncthreads();
+  const bool vecOut = (p.J & 3) == 0;
+  for (int e = threadIdx.x; e < T * T / 4; e += THREADS) {
+    const int r = e / (T / 4), q = (e - r * (T / 4)) * 4;
+    const float4 v = *reinterpret_cast<const float4 *>(part + r * PT + q);
+    const int i = i0 + r, j = j0 + q;
+    if (i >= p.I || j >= p.J) continue;
+    const size_t at = (size_t)i * p.J + j;
+    float z[4] = {v.x, v.y, v.z, v.w}, y[4];
+    const int m = p.J - j < 4 ? p.J - j : 4;
+    if (p.bias)
+      for (int k = 0; k < m; k++) z[k] += p.bias[j + k];
+#pragma unroll
+    for (int k = 0; k < 4; k++) y[k] = p.act ? z[k] * sigmoid(z[k]) : z[k];
+    if (vecOut && VEC) {
+      *reinterpret_cast<float4 *>(p.C + at) = make_float4(z[0], z[1], z[2], z[3]);
+      if (p.Yf) *reinterpret_cast<float4 *>(p.Yf + at) = make_float4(y[0], y[1], y[2], y[3]);
+      if (p.Y)
+        *reinterpret_cast<uint2 *>(p.Y + at) = make_uint2((uint32_t)f2bf(y[0]) | ((uint32_t)f2bf(y[1]) << 16),
+                                                          (uint32_t)f2bf(y[2]) | ((uint32_t)f2bf(y[3]) << 16));
+    } else {
+      for (int k = 0; k < m; k++) {
+        p.C[at + k] = z[k];
+        if (p.Yf) p.Yf[at + k] = y[k];
+        if (p.Y) p.Y[at + k] = f2bf(y[k]);
       }
     }
-}
-
-// Z = C + bias (in place), Y = act(Z) in BF16 and optionally FP32.
-__global__ void k_bias_act(int M, int N, float *Z, const float *bias, int act, uint16_t *Y, float *Yf) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= M * N) return;
-  const float z = Z[t] + (bias ? bias[t % N] : 0.f);
-  Z[t] = z;
-  const float y = act ? z * sigmoid(z) : z;
-  if (Y) Y[t] = f2bf(y);
-  if (Yf) Yf[t] = y;
-}
-
-// dZ = dY act'(Z): FP32 copy (for db) and BF16 copy (for the products).
-__global__ void k_act_grad(int M, int N, const float *dY, const float *Z, int act, float *dZ, uint16_t *dZb) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= M * N) return;
-  float g = dY[t];
-  if (act) {
-    const float z = Z[t], s = sigmoid(z);
-    g *= s * (1.f + z * (1.f - s));
   }
-  dZ[t] = g;
-  dZb[t] = f2bf(g);
 }
 
-// db[n] = sum_m dZ[m,n]: 32 columns per 256-thread CTA, 8 row slices per
-// column (slice r sums rows r, r+8, ... in order), the slices then added in a
-// fixed tree order -- parallel and reproducible.
-__global__ void __launch_bounds__(256) k_colsum(int M, int N, const float *dZ, float *db) {
+// dZ = dY act'(Z): FP32 copy, BF16 copy (for the products) and its column
+// sums db[n] = sum_m dZ[m,n].  A CTA owns 32 columns and takes 128 rows at a
+// time with all its threads; the sum of a column is 8 slices (slice r adds
+// rows r, r+8, ... in order) added in a fixed tree, so it is reproducible.
+constexpr int kGradRows = 128;
+__global__ void __launch_bounds__(1024) k_act_grad(int M, int N, const float *dY, const float *Z, int act, float *dZ,
+                                                   uint16_t *dZb, float *db) {
+  pdl_wait();
+  __shared__ float tile[kGradRows][33];
   __shared__ float part[8][33];
   const int c = threadIdx.x & 31, r = threadIdx.x >> 5;
   const int n = blockIdx.x * 32 + c;
   float s = 0.f;
-  if (n < N)
-    for (int m = r; m < M; m += 8) s += dZ[(size_t)m * N + n];
-  part[r][c] = s;
+  for (int m0 = 0; m0 < M; m0 += kGradRows) {
+#pragma unroll
+    for (int k = 0; k < kGradRows / 32; k++) {
+      const int row = r + 32 * k, m = m0 + row;
+      if (n < N && m < M) {
+        const size_t t = (size_t)m * N + n;
+        float g = dY[t];
+        if (act) {
+          const float z = Z[t], sg = sigmoid(z);
+          g *= sg * (1.f + z * (1.f - sg));
+        }
+        dZ[t] = g;
+        dZb[t] = f2bf(g);
+        tile[row][c] = g;
+      }
+    }
+    __syncthreads();
+    const int rows = M - m0 < kGradRows ? M - m0 : kGradRows;
+    if (r < 8 && n < N)
+      for (int row = r; row < rows; row += 8) s += tile[row][c];
+    __syncthreads();
+  }
+  if (r < 8) part[r][c] = s;
   __syncthreads();
   if (r == 0 && n < N)
     db[n] = ((part[0][c] + part[1][c]) + (part[2][c] + part[3][c])) +
             ((part[4][c] + part[5][c]) + (part[6][c] + part[7][c]));
 }
 
-// One CTA: loss and dY of the weighted mean squared error, summed in a fixed order.
-__global__ void k_mse(int M, int N, const float *Y, const float *T, const float *w, const float *we, float *dY,
-                      double *loss) {
-  __shared__ double red[1024];
-  double s = 0.0;
+// Loss and dY of the weighted mean squared error: one cluster of 8 CTAs, each
+// thread's terms, the threads of a CTA and the CTAs added in a fixed order.
+constexpr int kMseCtas = 8;
+__global__ void __launch_bounds__(1024) k_mse(int M, int N, const float *Y, const float *T, const float *w,
+                                              const float *we, float *dY, double *loss) {
+  pdl_wait();
+  __shared__ double red[33];
   const float inv = 1.f / (float)M;
-  for (int t = threadIdx.x; t < M * N; t += blockDim.x) {
+  const int n = M * N;
+  double s = 0.0;
+  for (int t = blockIdx.z * 1024 + threadIdx.x; t < n; t += kMseCtas * 1024) {
     const float wn = (w ? w[t % N] : 1.f) * (we ? we[t] : 1.f);
     const float d = Y[t] - T[t];
     dY[t] = 2.f * wn * d * inv;
     s += (double)wn * d * d;
   }
-  red[threadIdx.x] = s;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
+  if (threadIdx.x < 32) {
+    s = red[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+    if (threadIdx.x == 0) red[32] = s;
   }
-  if (threadIdx.x == 0 && loss) *loss = red[0] / M;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  if (blockIdx.z == 0 && threadIdx.x == 0 && loss) {
+    double a = 0.0;
+    for (int k = 0; k < kMseCtas; k++) a += *cluster.map_shared_rank(&red[32], k);
+    *loss = a / M;
+  }
+  cluster.sync();
 }
 
+__device__ __forceinline__ float adam_one(float w, float gt, float &m, float &v, float lr, float b1, float b2,
+                                          float eps, float wd, float c1, float c2) {
+  m = b1 * m + (1.f - b1) * gt;
+  v = b2 * v + (1.f - b2) * gt * gt;
+  return w - lr * ((m / c1) / (sqrtf(v / c2) + eps) + wd * w);
+}
+
+// VEC: four parameters per thread (n a multiple of 4, all arrays aligned).
+template <bool VEC>
 __global__ void k_adam(int n, float *master, uint16_t *wb, const float *g, float *m, float *v, float lr, float b1,
                        float b2, float eps, float wd, float c1, float c2) {
+  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const float gt = g[t];
-  const float mt = b1 * m[t] + (1.f - b1) * gt;
-  const float vt = b2 * v[t] + (1.f - b2) * gt * gt;
-  m[t] = mt;
-  v[t] = vt;
-  float w = master[t];
-  w -= lr * ((mt / c1) / (sqrtf(vt / c2) + eps) + wd * w);
-  master[t] = w;
-  if (wb) wb[t] = f2bf(w);
+  if (VEC) {
+    if (4 * (long long)t >= n) return;
+    float4 w4 = reinterpret_cast<float4 *>(master)[t], m4 = reinterpret_cast<float4 *>(m)[t];
+    float4 v4 = reinterpret_cast<float4 *>(v)[t];
+    const float4 g4 = reinterpret_cast<const float4 *>(g)[t];
+    w4.x = adam_one(w4.x, g4.x, m4.x, v4.x, lr, b1, b2, eps, wd, c1, c2);
+    w4.y = adam_one(w4.y, g4.y, m4.y, v4.y, lr, b1, b2, eps, wd, c1, c2);
+    w4.z = adam_one(w4.z, g4.z, m4.z, v4.z, lr, b1, b2, eps, wd, c1, c2);
+    w4.w = adam_one(w4.w, g4.w, m4.w, v4.w, lr, b1, b2, eps, wd, c1, c2);
+    reinterpret_cast<float4 *>(m)[t] = m4;
+    reinterpret_cast<float4 *>(v)[t] = v4;
+    reinterpret_cast<float4 *>(master)[t] = w4;
+    if (wb)
+      reinterpret_cast<uint2 *>(wb)[t] = make_uint2((uint32_t)f2bf(w4.x) | ((uint32_t)f2bf(w4.y) << 16),
+                                                    (uint32_t)f2bf(w4.z) | ((uint32_t)f2bf(w4.w) << 16));
+  } else {
+    if (t >= n) return;
+    float mt = m[t], vt = v[t];
+    const float w = adam_one(master[t], g[t], mt, vt, lr, b1, b2, eps, wd, c1, c2);
+    m[t] = mt;
+    v[t] = vt;
+    master[t] = w;
+    if (wb) wb[t] = f2bf(w);
+  }
 }
 
+template <bool VEC>
 __global__ void k_to_bf16(int n, const float *x, uint16_t *y) {
+  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) y[t] = f2bf(x[t]);
+  if (VEC) {
+    if (4 * (long long)t >= n) return;
+    const float4 v = reinterpret_cast<const float4 *>(x)[t];
+    reinterpret_cast<uint2 *>(y)[t] = make_uint2((uint32_t)f2bf(v.x) | ((uint32_t)f2bf(v.y) << 16),
+                                                 (uint32_t)f2bf(v.z) | ((uint32_t)f2bf(v.w) << 16));
+  } else if (t < n) {
+    y[t] = f2bf(x[t]);
+  }
 }
 
 inline int grid1(long long n) { return (int)((n + 255) / 256); }
+inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+inline bool aligned8(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; }
 
-int gemm(int I, int J, int Lk, const uint16_t *A, long long sai, long long sal, const uint16_t *B, long long sbl,
-         long long sbj, float *C, cudaStream_t s) {
-  dim3 grid((J + kT - 1) / kT, (I + kT - 1) / kT);
-  k_gemm_bf16<<<grid, 256, 0, s>>>(I, J, Lk, A, sai, sal, B, sbl, sbj, C);
+template <int T, bool VEC>
+int gemm_t(Products &ps, int count, cudaStream_t s) {
+  constexpr size_t smem = sizeof(uint16_t) * 2 * stages<T>() * stage_elems<T>();
+  static_assert(smem >= sizeof(float) * T * (T + 4), "the tile fits the staging buffers");
+  int tiles = 0;
+  for (int k = 0; k < 2; k++) {
+    Product &p = ps.p[k];
+    if (k >= count) {
+      p = ps.p[0];
+      p.tiles = 0;
+      continue;
+    }
+    p.tilesJ = (p.J + T - 1) / T;
+    p.tiles = (p.I + T - 1) / T * p.tilesJ;
+    tiles += p.tiles;
+  }
+  auto k = k_gemm_bf16<T, VEC>;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return BNB_ERR_CUDA;
+  launch_pdl(k, tiles, T == 64 ? 256 : 128, smem, s, ps);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
+}
+
+int gemm(Products &ps, int count, cudaStream_t s) {
+  long long tiles64 = 0;
+  bool vec = true;
+  for (int k = 0; k < count; k++) {
+    const Product &p = ps.p[k];
+    tiles64 += (long long)((p.I + 63) / 64) * ((p.J + 63) / 64);
+    vec = vec && (p.lastA ? p.I : p.L) % 8 == 0 && (p.lastB ? p.J : p.L) % 8 == 0 && aligned16(p.A) &&
+          aligned16(p.B) && aligned16(p.C) && aligned16(p.Yf) && aligned8(p.Y);
+  }
+  if (tiles64 >= 74) return vec ? gemm_t<64, true>(ps, count, s) : gemm_t<64, false>(ps, count, s);
+  return vec ? gemm_t<32, true>(ps, count, s) : gemm_t<32, false>(ps, count, s);
 }
 
 }  // namespace
@@ -196,11 +419,10 @@ extern "C" int bnb_mlp_linear_forward(int M, int N, int K, const uint16_t *X, co
   if (M < 0 || N < 0 || K < 0 || !X || !W || !Z || (act != 0 && act != 1)) return BNB_ERR_ARG;
   if ((long long)M * N >= (1ll << 31)) return BNB_ERR_ARG;
   if (M == 0 || N == 0) return BNB_OK;
-  cudaStream_t s = (cudaStream_t)stream;
-  int rc = gemm(M, N, K, X, K, 1, W, 1, K, Z, s);  // Z[m,n] = sum_k X[m,k] W[n,k]
-  if (rc) return rc;
-  k_bias_act<<<grid1((long long)M * N), 256, 0, s>>>(M, N, Z, bias, act, Y, Yf);
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
+  Products ps{};
+  // Z[m,n] = sum_k X[m,k] W[n,k]
+  ps.p[0] = Product{X, W, M, N, K, 0, 0, 0, 0, Z, bias, act, Y, Yf};
+  return gemm(ps, 1, (cudaStream_t)stream);
 }
 
 extern "C" int bnb_mlp_linear_backward(int M, int N, int K, const float *dY, const float *Z, int act,
@@ -211,21 +433,20 @@ extern "C" int bnb_mlp_linear_backward(int M, int N, int K, const float *dY, con
   if ((long long)M * N >= (1ll << 31) || (long long)M * K >= (1ll << 31)) return BNB_ERR_ARG;
   if (M == 0 || N == 0) return BNB_OK;
   cudaStream_t s = (cudaStream_t)stream;
-  k_act_grad<<<grid1((long long)M * N), 256, 0, s>>>(M, N, dY, Z, act, dZ, dZb);
-  k_colsum<<<(N + 31) / 32, 256, 0, s>>>(M, N, dZ, db);
-  int rc = gemm(N, K, M, dZb, 1, N, X, K, 1, dW, s);  // dW[n,k] = sum_m dZ[m,n] X[m,k]
-  if (rc) return rc;
-  if (dX) {
-    rc = gemm(M, K, N, dZb, N, 1, W, K, 1, dX, s);  // dX[m,k] = sum_n dZ[m,n] W[n,k]
-    if (rc) return rc;
-  }
-  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
+  launch_pdl(k_act_grad, (N + 31) / 32, 1024, 0, s, M, N, dY, Z, act, dZ, dZb, db);
+  if (cudaGetLastError() != cudaSuccess) return BNB_ERR_CUDA;
+  if (K == 0) return BNB_OK;
+  Products ps{};
+  ps.p[0] = Product{dZb, X, N, K, M, 1, 1, 0, 0, dW, nullptr, 0, nullptr, nullptr};  // dW[n,k] = sum_m dZ[m,n] X[m,k]
+  ps.p[1] = Product{dZb, W, M, K, N, 0, 1, 0, 0, dX, nullptr, 0, nullptr, nullptr};  // dX[m,k] = sum_n dZ[m,n] W[n,k]
+  return gemm(ps, dX ? 2 : 1, s);
 }
 
 extern "C" int bnb_mlp_mse(int M, int N, const float *Y, const float *T, const float *weight,
                            const float *elemWeight, float *dY, double *loss, void *stream) {
   if (M <= 0 || N <= 0 || !Y || !T || !dY) return BNB_ERR_ARG;
-  k_mse<<<1, 1024, 0, (cudaStream_t)stream>>>(M, N, Y, T, weight, elemWeight, dY, loss);
+  launch_pdl(k_mse, ClusterGrid{dim3(1, 1, kMseCtas), kMseCtas}, 1024, 0, (cudaStream_t)stream, M, N, Y, T, weight,
+             elemWeight, dY, loss);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
 
@@ -235,14 +456,23 @@ extern "C" int bnb_mlp_adam(int n, float *master, uint16_t *weightBf16, const fl
   if (n < 0 || step < 1 || (n > 0 && (!master || !grad || !m || !v))) return BNB_ERR_ARG;
   if (n == 0) return BNB_OK;
   const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
-  k_adam<<<grid1(n), 256, 0, (cudaStream_t)stream>>>(n, master, weightBf16, grad, m, v, lr, beta1, beta2, eps,
-                                                     weightDecay, c1, c2);
+  const bool vec = n % 4 == 0 && aligned16(master) && aligned16(grad) && aligned16(m) && aligned16(v) &&
+                   aligned8(weightBf16);
+  if (vec)
+    launch_pdl(k_adam<true>, grid1(n / 4), 256, 0, (cudaStream_t)stream, n, master, weightBf16, grad, m, v, lr, beta1,
+               beta2, eps, weightDecay, c1, c2);
+  else
+    launch_pdl(k_adam<false>, grid1(n), 256, 0, (cudaStream_t)stream, n, master, weightBf16, grad, m, v, lr, beta1,
+               beta2, eps, weightDecay, c1, c2);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
 
 extern "C" int bnb_to_bf16(int n, const float *x, uint16_t *y, void *stream) {
   if (n < 0 || (n > 0 && (!x || !y))) return BNB_ERR_ARG;
   if (n == 0) return BNB_OK;
-  k_to_bf16<<<grid1(n), 256, 0, (cudaStream_t)stream>>>(n, x, y);
+  if (n % 4 == 0 && aligned16(x) && aligned8(y))
+    launch_pdl(k_to_bf16<true>, grid1(n / 4), 256, 0, (cudaStream_t)stream, n, x, y);
+  else
+    launch_pdl(k_to_bf16<false>, grid1(n), 256, 0, (cudaStream_t)stream, n, x, y);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }

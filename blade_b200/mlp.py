@@ -27,16 +27,32 @@ class BF16MLP:
         self.max_batch = max_batch
         rng = np.random.default_rng(seed)
         f32, bf = torch.float32, torch.int16
+        # One buffer each for the parameters, their gradients, the Adam moments
+        # and the BF16 copies: all weights, then all biases, every tensor
+        # padded to 64 elements; the lists below are views.  The optimizer and
+        # the BF16 conversion are then one launch over all layers.
+        pad = lambda n: (n + 63) // 64 * 64
+        layers = list(zip(self.sizes[:-1], self.sizes[1:]))
+        self._nW = sum(pad(N * K) for K, N in layers)
+        total = self._nW + sum(pad(N) for _, N in layers)
+        self._p, self._g, self._m, self._v = (torch.zeros(total, dtype=f32, device=self.dev) for _ in range(4))
+        self._pb = torch.zeros(total, dtype=bf, device=self.dev)
         self.W, self.Wb, self.b, self.mW, self.vW, self.mb, self.vb, self.gW, self.gb = ([] for _ in range(9))
-        for K, N in zip(self.sizes[:-1], self.sizes[1:]):
+        oW, ob = 0, self._nW
+        for K, N in layers:
             bound = np.sqrt(6.0 / K) if len(self.W) < len(self.sizes) - 2 else np.sqrt(1.0 / K)
             w = rng.uniform(-bound, bound, (N, K)).astype(np.float32)
-            self.W.append(torch.from_numpy(w).to(self.dev))
-            self.Wb.append(torch.empty(N * K, dtype=bf, device=self.dev))
-            self.b.append(torch.zeros(N, dtype=f32, device=self.dev))
-            for lst, n in ((self.mW, N * K), (self.vW, N * K), (self.gW, N * K), (self.mb, N), (self.vb, N),
-                           (self.gb, N)):
-                lst.append(torch.zeros(n, dtype=f32, device=self.dev))
+            self.W.append(self._p[oW:oW + N * K].view(N, K))
+            self.W[-1].copy_(torch.from_numpy(w))
+            self.Wb.append(self._pb[oW:oW + N * K])
+            self.b.append(self._p[ob:ob + N])
+            for lst, src, o, n in ((self.mW, self._m, oW, N * K), (self.vW, self._v, oW, N * K),
+                                   (self.gW, self._g, oW, N * K), (self.mb, self._m, ob, N),
+                                   (self.vb, self._v, ob, N), (self.gb, self._g, ob, N)):
+                lst.append(src[o:o + n])
+            oW += pad(N * K)
+            ob += pad(N)
+        self._views = [list(x) for x in (self.W, self.Wb, self.b, self.gW, self.gb, self.mW, self.mb, self.vW, self.vb)]
         self._sync_bf16()
         M = max_batch
         self.xb = torch.empty(M * self.sizes[0], dtype=bf, device=self.dev)
@@ -53,7 +69,16 @@ class BF16MLP:
     def _s(self):
         return C.c_void_p(self.torch.cuda.current_stream().cuda_stream)
 
+    def _whole(self):
+        """True while the lists hold the views made by __init__ (a caller may
+        put tensors of its own in them, such as clipped gradients)."""
+        lists = (self.W, self.Wb, self.b, self.gW, self.gb, self.mW, self.mb, self.vW, self.vb)
+        return all(a is b for x, y in zip(lists, self._views) for a, b in zip(x, y))
+
     def _sync_bf16(self):
+        if self._whole():
+            _lib.call("bnb_to_bf16", self._p.numel(), _p(self._p), _p(self._pb), self._s())
+            return
         for W, Wb in zip(self.W, self.Wb):
             _lib.call("bnb_to_bf16", W.numel(), _p(W), _p(Wb), self._s())
 
@@ -106,11 +131,19 @@ class BF16MLP:
     def adam_step(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0):
         self.step_count += 1
         s = self._s()
-        for l in range(self.n_layers):
-            _lib.call("bnb_mlp_adam", self.W[l].numel(), _p(self.W[l]), _p(self.Wb[l]), _p(self.gW[l]),
-                      _p(self.mW[l]), _p(self.vW[l]), lr, beta1, beta2, eps, weight_decay, self.step_count, s)
-            _lib.call("bnb_mlp_adam", self.b[l].numel(), _p(self.b[l]), None, _p(self.gb[l]), _p(self.mb[l]),
-                      _p(self.vb[l]), lr, beta1, beta2, eps, 0.0, self.step_count, s)
+        # weight decay acts on the weights alone: with it, the biases are a second launch
+        if not self._whole():
+            for l in range(self.n_layers):
+                _lib.call("bnb_mlp_adam", self.W[l].numel(), _p(self.W[l]), _p(self.Wb[l]), _p(self.gW[l]),
+                          _p(self.mW[l]), _p(self.vW[l]), lr, beta1, beta2, eps, weight_decay, self.step_count, s)
+                _lib.call("bnb_mlp_adam", self.b[l].numel(), _p(self.b[l]), None, _p(self.gb[l]), _p(self.mb[l]),
+                          _p(self.vb[l]), lr, beta1, beta2, eps, 0.0, self.step_count, s)
+            return
+        parts = [(0, self._p.numel(), 0.0)] if weight_decay == 0.0 else \
+            [(0, self._nW, weight_decay), (self._nW, self._p.numel(), 0.0)]
+        for a, b, wd in parts:
+            _lib.call("bnb_mlp_adam", b - a, _p(self._p[a:b]), _p(self._pb[a:b]), _p(self._g[a:b]), _p(self._m[a:b]),
+                      _p(self._v[a:b]), lr, beta1, beta2, eps, wd, self.step_count, s)
 
     def train_step(self, x, target, weight=None, lr=1e-3, elem_weight=None):
         loss = self.loss_grad(x, target, weight, elem_weight)

@@ -129,3 +129,70 @@ def test_training_reduces_loss(cuda):
         net.train_step(X[k:k + 128], T[k:k + 128], lr=3e-3)
     last = float(net.loss_grad(X[:128], T[:128]).cpu()[0])
     assert last < 0.1 * first
+
+
+# Tile edges (32 and 64), ragged and 16-byte-aligned extents, one element, more
+# chunks than the ring holds, enough tiles for the 64-wide kernel.
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 8, 8), (3, 5, 7), (32, 32, 64), (33, 31, 65), (64, 40, 264),
+                                   (65, 128, 1664), (256, 256, 1664), (7, 24, 2056), (600, 584, 72), (577, 600, 63)])
+def test_products_at_tile_edges(cuda, M, N, K):
+    rng = np.random.default_rng(M + N + K)
+    X, W = _bf16(rng.normal(size=(M, K))), _bf16(rng.normal(0, 0.1, (N, K)))
+    b = torch.as_tensor(rng.normal(0, 0.1, N).astype(np.float32), device="cuda")
+    Z, Yf, dZ = (torch.full((M * N,), float("nan"), device="cuda") for _ in range(3))
+    Yb, dZb = (torch.empty(M * N, dtype=torch.int16, device="cuda") for _ in range(2))
+    dX, dW, db = (torch.full((n,), float("nan"), device="cuda") for n in (M * K, N * K, N))
+    dY = torch.as_tensor(rng.normal(size=(M, N)).astype(np.float32), device="cuda")
+    _lib.call("bnb_mlp_linear_forward", M, N, K, _p(X), _p(W), _p(b), 1, _p(Z), _p(Yb), _p(Yf), _s())
+    _lib.call("bnb_mlp_linear_backward", M, N, K, _p(dY), _p(Z), 1, _p(X), _p(W), _p(dZ), _p(dZb), _p(dX), _p(dW),
+              _p(db), _s())
+    Xh, Wh = _decode(X, (M, K)), _decode(W, (N, K))
+    Zo, Yo = mo.linear_forward(Xh, Wh, b.cpu().numpy().astype(np.float64), 1)
+    # FP32 accumulation of n products: at most n 2^-24 of sum |x||w| (BF16 products are exact in FP32)
+    lim = lambda a, bt, n: (n + 2) * 2.0 ** -24 * (np.abs(a) @ np.abs(bt)) + 1e-6
+    Zg = Z.cpu().numpy().reshape(M, N).astype(np.float64)
+    assert (np.abs(Zg - Zo) <= lim(Xh, Wh.T, K)).all()
+    assert _rel(Yf.cpu().numpy().reshape(M, N), Yo) < ACC_TOL
+    np.testing.assert_array_equal(_decode(Yb, (M, N)), mo.bf16_round(Yf.cpu().numpy().reshape(M, N)))
+    dZo, _, _, _, dbo = mo.linear_backward(dY.cpu().numpy().astype(np.float64), Zg, 1, Xh, Wh)
+    assert _rel(dZ.cpu().numpy().reshape(M, N), dZo) < ACC_TOL
+    assert (np.abs(db.cpu().numpy() - dbo) <= (M + 8) * 2.0 ** -24 * np.abs(dZo).sum(0) + 1e-6).all()
+    dZh = _decode(dZb, (M, N))
+    assert (np.abs(dW.cpu().numpy().reshape(N, K) - dZh.T @ Xh) <= lim(dZh.T, Xh, M)).all()
+    assert (np.abs(dX.cpu().numpy().reshape(M, K) - dZh @ Wh) <= lim(dZh, Wh, N)).all()
+
+
+@pytest.mark.parametrize("M,N", [(1, 1), (5, 33), (256, 128), (300, 130)])
+def test_mse_matches_oracle(cuda, M, N):
+    rng = np.random.default_rng(M * N)
+    y, t, we = (rng.normal(size=(M, N)).astype(np.float32) for _ in range(3))
+    w = rng.uniform(0.5, 1.5, N).astype(np.float32)
+    dev = [torch.as_tensor(a, device="cuda") for a in (y, t, w, we)]
+    dY = torch.empty(M * N, device="cuda")
+    loss = torch.zeros(1, dtype=torch.float64, device="cuda")
+    _lib.call("bnb_mlp_mse", M, N, *[_p(a) for a in dev], _p(dY), _p(loss), _s())
+    ww = w.astype(np.float64) * we
+    d = y.astype(np.float64) - t
+    np.testing.assert_allclose(dY.cpu().numpy().reshape(M, N), 2 * ww * d / M, rtol=1e-5, atol=1e-7)
+    # each term's weight and difference are rounded to FP32
+    assert abs(float(loss.cpu()[0]) - (ww * d * d).sum() / M) <= 4 * 2.0 ** -23 * (np.abs(ww) * d * d).sum() / M
+
+
+def test_adam_step_takes_the_callers_gradients(cuda):
+    """One optimizer launch over all layers equals the layer-by-layer update,
+    and tensors that a caller puts into the lists are the ones that count."""
+    a, b = BF16MLP([72, 40, 10], max_batch=16, seed=3), BF16MLP([72, 40, 10], max_batch=16, seed=3)
+    x, t = torch.randn(16, 72, device="cuda"), torch.randn(16, 10, device="cuda")
+    for net, wd in ((a, 0.0), (b, 0.0)):
+        net.loss_grad(x, t)
+    b.gW[0] = b.gW[0].clone()                       # the same values in another tensor
+    for wd in (0.0, 0.01):
+        a.adam_step(weight_decay=wd)
+        b.adam_step(weight_decay=wd)
+        for l in range(2):
+            assert torch.equal(a.W[l], b.W[l]) and torch.equal(a.b[l], b.b[l]) and torch.equal(a.Wb[l], b.Wb[l])
+    before = b.W[0].clone()
+    b.gW[0].zero_()
+    b.mW[0].zero_()
+    b.adam_step()
+    assert torch.equal(b.W[0], before)
