@@ -18,7 +18,8 @@ namespace bnb {
 
 constexpr int kNumShifts = 14;        // own image + 13 half-shell images
 constexpr int kExclBlk = 16;          // exclusion-partner blocks listed per block
-constexpr int kTilesPerWork = 8;      // default candidate tiles per pair-kernel work item
+constexpr int kTilesPerWork = 8;      // most candidate tiles per pair-kernel work item by default
+constexpr int kMinAutoTiles = 2;      // fewest by default (replica_tiles)
 constexpr int kMinTilesPerWork = 1;   // smallest setting (sizes the work-item capacity)
 constexpr int kTailItems = 2;         // full-size items' worth of tiles per i block in the tail levels
 constexpr int kMaxTableTypes = 64;    // LJ table kept in shared memory up to 64 types
@@ -65,6 +66,8 @@ struct RepInfo {          // per replica, device copy in Dev::rep
   int divX, divY;
   int lamStart, lamCount;
   float tric[3];          // B_x, C_x, C_y
+  int tilesPerWork;       // candidate tiles per work item (1..32)
+  int tailTiles;          // last candidate tiles of each i block that go to the tail levels
   float4 shift[14];       // image shift vectors by shift code (kNumShifts)
 };
 
@@ -108,8 +111,6 @@ struct Counters {
 struct Dev {
   // --- static topology (set_topology) -------------------------------------
   int N, R, nTypes, ljCombine, lamTotal;
-  int tilesPerWork;        // candidate tiles per work item (tuning knob, 1..32)
-  int tailTiles;           // last candidate tiles of each i block that go to the tail levels
   RepInfo *rep;            // [R]
   int *atomRep;            // [N]
   float *atomQ;            // [N] charge * sqrt(kElectric)
@@ -138,6 +139,7 @@ struct Dev {
   int *atomSlot;           // [N]
   float *slotQ;            // [32*maxBlocks]
   int *slotType;           // [32*maxBlocks]
+  float2 *slotLj;          // [32*maxBlocks] combine mode: ljType of the slot's type
   int *slotSiteBlock;      // [32*maxBlocks]
   uint32_t *colKey;        // [6*totalCols] column AABB (union of its blocks) as order-preserving keys
   int *exclBlk;            // [maxBlocks*kExclBlk] distinct blocks holding excluded partners
@@ -147,7 +149,7 @@ struct Dev {
   int4 *cand;              // [capCand] (jBlock, shiftCode, maskIdx, iBlock)
   int *candFlag;           // [capCand]
   int *candMaskOff;        // [capCand+1]
-  uint32_t *masks;         // [capMask*32]
+  uint32_t *masks;         // [capMask*32] word of j atom l: bit i clear = excluded from i atom i
   int *candStart;          // [maxBlocks+1]
   int2 *work;              // [capWork] (iBlock | tiles << 22, candidate start)
   unsigned int *itemCost;  // [capWork] clock cycles of each work item in the last pair launch
@@ -156,6 +158,7 @@ struct Dev {
   // --- per-step buffers -----------------------------------------------------
   float4 *xyzq;            // [32*maxBlocks]
   float4 *bmin, *bmax;     // [maxBlocks]
+  float4 *hmin, *hmax;     // [2*maxBlocks] AABBs of the blocks' halves (slots 0-15, 16-31)
   long long *accF;         // [3*32*maxBlocks] SoA fixed-point dU/dx per slot
   long long *accL;         // [lamTotal]
   long long *accE;         // [1]

@@ -52,7 +52,8 @@ struct bnb_handle {
   int resTiles = 0, resMasks = 0, resWork = 0;
   bool reserveDirty = false;
   int tilesPerWork = bnb::kTilesPerWork, ctasPerSM = 0;  // tuning (bnb_set_tuning / bnb_autotune)
-  int tailItems = bnb::kTailItems;
+  int tailItems = 0;
+  bool tuned = false;  // the caller's tuning; until then every replica has its own (replica_tiles)
   int smCount = 0;
   bool counting = false;
   bool orderPending = false;  // sort the work items by cost after the next pair launch
@@ -196,7 +197,8 @@ int alloc_list(bnb_handle *h) {
   size_t o_bucket = a.take<int>(N), o_sorted = a.take<int>(N);
   size_t o_bb = a.take<int>(MB + 1), o_brep = a.take<int>(MB), o_rbs = a.take<int>(h->R + 1);
   size_t o_slotA = a.take<int>(32 * MB), o_atomSlot = a.take<int>(N), o_slotQ = a.take<float>(32 * MB),
-         o_slotT = a.take<int>(32 * MB), o_slotSB = a.take<int>(32 * MB);
+         o_slotT = a.take<int>(32 * MB), o_slotSB = a.take<int>(32 * MB),
+         o_slotLj = a.take<float2>(32 * (size_t)MB);
   size_t o_ckey = a.take<uint32_t>(6 * (size_t)C), o_eb = a.take<int>(bnb::kExclBlk * MB),
          o_ebc = a.take<int>(MB);
   size_t o_cullC = a.take<int>(MB * bnb::kNumShifts), o_cullO = a.take<int>(MB * bnb::kNumShifts + 1);
@@ -207,6 +209,7 @@ int alloc_list(bnb_handle *h) {
          o_order = a.take<int>(h->capWork);
   size_t o_part = a.take<int>(4096);
   size_t o_xyzq = a.take<float4>(32 * MB), o_bmin = a.take<float4>(MB), o_bmax = a.take<float4>(MB);
+  size_t o_hmin = a.take<float4>(2 * (size_t)MB), o_hmax = a.take<float4>(2 * (size_t)MB);
   size_t o_acc = a.take<long long>(3 * 32 * (size_t)MB);
   void *base = nullptr;
   if (!ok(cudaMalloc(&base, a.off))) return BNB_ERR_CUDA;
@@ -231,6 +234,7 @@ int alloc_list(bnb_handle *h) {
   d.slotQ = (float *)(b + o_slotQ);
   d.slotType = (int *)(b + o_slotT);
   d.slotSiteBlock = (int *)(b + o_slotSB);
+  d.slotLj = (float2 *)(b + o_slotLj);
   d.colKey = (uint32_t *)(b + o_ckey);
   d.exclBlk = (int *)(b + o_eb);
   d.exclBlkCount = (int *)(b + o_ebc);
@@ -248,6 +252,8 @@ int alloc_list(bnb_handle *h) {
   d.xyzq = (float4 *)(b + o_xyzq);
   d.bmin = (float4 *)(b + o_bmin);
   d.bmax = (float4 *)(b + o_bmax);
+  d.hmin = (float4 *)(b + o_hmin);
+  d.hmax = (float4 *)(b + o_hmax);
   d.accF = (long long *)(b + o_acc);
   d.totalCols = C;
   d.maxBlocks = MB;
@@ -345,21 +351,40 @@ bool layout_columns(bnb_handle *h, const float *boxes) {
   return changed;
 }
 
+// Candidate tiles of one replica, estimated from its density and cutoff.
+double tiles_estimate(const bnb_handle *h, int r) {
+  const RepInfo &ri = h->rep[r];
+  const int n = h->atomCount[r];
+  if (n == 0) return 0;
+  const double vol = (double)ri.box[0] * ri.box[1] * ri.box[2], invDens = vol / n;
+  const double edge = std::cbrt(32 * invDens) + 2.0 * (h->p.rCut + h->p.cullPad);
+  return (0.75 * edge * edge * edge / (32 * invDens) + 16) * (n / 32 + 1);
+}
+
+// Default candidate tiles per work item of a replica: the largest power of two
+// in [2, 8] that still gives the 2,368 warps the pair kernel keeps resident
+// (148 SMs x 16) an item each, by the estimate above, so that a small system is
+// spread over the GPU and a large one pays each item's set-up and half-empty
+// last round less often.  The estimate exceeds the real count by 1.1 (648
+// atoms, 9 A) to 1.5 times (3,000, 12 A), hence the factor.  It depends on the replica
+// alone, so a replica gives the same bits alone and in a batch.  Pair kernel,
+// us, at 1 / 2 / 4 / 8 tiles an item: 648 atoms 15 / 16 / 20 / 28, 519 with
+// MSLD 19 / 25 / 34 / 56, 3,000 (12 A) 21 / 21 / 28 / 40, 20,577 (9 A)
+// 58 / 46 / 39 / 38, 23,558 (12 A) 105 / 82 / 70 / 66, 32 MSLD boxes of 690
+// atoms in a batch 100 / 80 / 68 / 75.
+int replica_tiles(const bnb_handle *h, int r) {
+  const double items = tiles_estimate(h, r) / 1.5;
+  int t = bnb::kMinAutoTiles;
+  while (t < bnb::kTilesPerWork && items >= 2.0 * t * 2368) t *= 2;
+  return t;
+}
+
 void estimate_capacities(bnb_handle *h, int &mb, long long &cand, long long &work, long long &mask) {
   mb = 0;
   cand = 0;
   for (int r = 0; r < h->R; r++) {
-    const RepInfo &ri = h->rep[r];
-    int n = h->atomCount[r];
-    int blocks = n / 32 + ri.nCols + 1;
-    mb += blocks;
-    if (n == 0) continue;
-    double vol = (double)ri.box[0] * ri.box[1] * ri.box[2];
-    double invDens = vol / n;
-    double approx = std::cbrt(32 * invDens);
-    double edge = approx + 2.0 * (h->p.rCut + h->p.cullPad);
-    double perBlock = 0.75 * edge * edge * edge / (32 * invDens) + 16;
-    cand += (long long)(perBlock * (n / 32 + 1)) + 14;
+    mb += h->atomCount[r] / 32 + h->rep[r].nCols + 1;
+    if (h->atomCount[r] > 0) cand += (long long)tiles_estimate(h, r) + 14;
   }
   work = cand / bnb::kMinTilesPerWork + mb + 16;
   mask = (long long)(4 * h->exclTotal + 1024) / 32 + 64;
@@ -641,8 +666,14 @@ int bnb_set_topology(bnb_handle *h, const bnb_nbond *nbonds, const int *typeCoun
 // taking small ones while the rest finish.  The split depends on the block's
 // own candidates only: an i atom's force is summed in FP32 over the tiles of
 // one item, so a replica gives the same bits alone and in a batch.
-static void set_tail(bnb_handle *h) {
-  h->d.tailTiles = h->tailItems * h->tilesPerWork;
+// Without a tuning of the caller's there is no tail: the longest-first order
+// balances the launches after a list's first (batch of 8 MSLD replicas: 182 us
+// a launch without, 190 with two items' worth; equal on the others).
+static void set_work_split(bnb_handle *h) {
+  for (int r = 0; r < h->R; r++) {
+    h->rep[r].tilesPerWork = h->tuned ? h->tilesPerWork : replica_tiles(h, r);
+    h->rep[r].tailTiles = h->tuned ? h->tailItems * h->tilesPerWork : 0;
+  }
 }
 
 int bnb_rebuild(bnb_handle *h, const float *position, const float *boxes, void *stream, int flags) {
@@ -675,12 +706,11 @@ int bnb_rebuild(bnb_handle *h, const float *position, const float *boxes, void *
     int rc = alloc_list(h);
     if (rc) return rc;
   }
+  set_work_split(h);
   int rc = upload_rep(h, s);
   if (rc) return rc;
   const float rcull = h->p.rCut + h->p.cullPad;
   const float rcull2 = rcull * rcull;
-  h->d.tilesPerWork = h->tilesPerWork;
-  set_tail(h);
   for (int attempt = 0; attempt < 12; attempt++) {
     const bool rec = h->prof && h->rebN < kProfSlots;
     if (rec) cudaEventRecord(h->rebEv[2 * h->rebN], s);
@@ -830,8 +860,13 @@ int bnb_set_tuning(bnb_handle *h, int tilesPerWork, int ctasPerSM, int tailItems
   if (!h || tilesPerWork < bnb::kMinTilesPerWork || tilesPerWork > 32 || ctasPerSM < 0 || ctasPerSM > 8 ||
       tailItems < 0 || tailItems > 8)
     return BNB_ERR_ARG;
-  // work items must be rebuilt
-  if (tilesPerWork != h->tilesPerWork || tailItems != h->tailItems) h->listBuilt = false;
+  // the work items must be rebuilt; a first call that names the general default
+  // or the choice in effect leaves a built list valid
+  int t0, l0;
+  bnb_get_tuning(h, &t0, nullptr, &l0);
+  const bool general = !h->tuned && tilesPerWork == bnb::kTilesPerWork && tailItems == bnb::kTailItems;
+  if (!general && (tilesPerWork != t0 || tailItems != l0)) h->listBuilt = false;
+  h->tuned = true;
   h->tilesPerWork = tilesPerWork;
   h->ctasPerSM = ctasPerSM;
   h->tailItems = tailItems;
@@ -840,7 +875,13 @@ int bnb_set_tuning(bnb_handle *h, int tilesPerWork, int ctasPerSM, int tailItems
 
 int bnb_get_tuning(bnb_handle *h, int *tilesPerWork, int *ctasPerSM, int *tailItems) {
   if (!h) return BNB_ERR_ARG;
-  if (tilesPerWork) *tilesPerWork = h->tilesPerWork;
+  if (tilesPerWork) {
+    *tilesPerWork = h->tilesPerWork;
+    if (!h->tuned && h->listArena) {  // the largest of the replicas' own
+      *tilesPerWork = 0;
+      for (const RepInfo &ri : h->rep) *tilesPerWork = std::max(*tilesPerWork, ri.tilesPerWork);
+    }
+  }
   if (ctasPerSM) *ctasPerSM = h->ctasPerSM;
   if (tailItems) *tailItems = h->tailItems;
   return BNB_OK;
@@ -966,7 +1007,16 @@ int bnb_get_list(bnb_handle *h, void *stream, int *wrap, int *blockBounds, int *
       if (candMask) candMask[c] = t[c].z;
     }
   }
-  dn(masks, d.masks, sizeof(uint32_t) * 32 * (size_t)M);
+  if (masks && M) {  // the device keeps a word per j atom; the export has a row per i atom
+    std::vector<uint32_t> t(32 * (size_t)M);
+    dn(t.data(), d.masks, sizeof(uint32_t) * t.size());
+    for (int m = 0; m < M; m++)
+      for (int i = 0; i < 32; i++) {
+        uint32_t row = 0;
+        for (int j = 0; j < 32; j++) row |= ((t[32 * (size_t)m + j] >> i) & 1u) << j;
+        masks[32 * (size_t)m + i] = row;
+      }
+  }
   return good ? BNB_OK : BNB_ERR_CUDA;
 }
 

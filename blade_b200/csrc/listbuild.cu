@@ -391,12 +391,15 @@ __global__ void k_slots(Dev d) {
     d.slotAtom[t] = a;
     d.atomSlot[a] = t;
     d.slotQ[t] = d.atomQ[a];
-    d.slotType[t] = d.atomType[a];
+    const int type = d.atomType[a];
+    d.slotType[t] = type;
+    if (d.ljCombine) d.slotLj[t] = d.ljType[type];
     d.slotSiteBlock[t] = d.atomSiteBlock[a];
   } else {
     d.slotAtom[t] = -1;
     d.slotQ[t] = 0.0f;
     d.slotType[t] = 0;
+    if (d.ljCombine) d.slotLj[t] = make_float2(0.f, 0.f);
     d.slotSiteBlock[t] = 0;
   }
 }
@@ -416,7 +419,7 @@ __global__ void k_pack(Dev d, const float *__restrict__ pos, bool columns) {
   if (b >= d.ctr->blockCount) return;
   int a = d.slotAtom[t];
   const RepInfo &ri = d.rep[d.blockRep[b]];
-  float3 p = make_float3(0.f, 0.f, 0.f);
+  float3 p = make_float3(1.0e18f, 0.f, 0.f);  // empty slot: outside every cutoff (k_pair)
   float3 mn = make_float3(INFINITY, INFINITY, INFINITY);
   float3 mx = make_float3(-INFINITY, -INFINITY, -INFINITY);
   if (a >= 0) {
@@ -431,7 +434,11 @@ __global__ void k_pack(Dev d, const float *__restrict__ pos, bool columns) {
   }
   d.xyzq[t] = make_float4(p.x, p.y, p.z, d.slotQ[t]);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = 1; o < 32; o <<= 1) {
+    if (o == 16 && (t & 15) == 0) {  // the halves' own boxes (k_pair)
+      d.hmin[t >> 4] = make_float4(mn.x, mn.y, mn.z, 0.f);
+      d.hmax[t >> 4] = make_float4(mx.x, mx.y, mx.z, 0.f);
+    }
     mn.x = fminf(mn.x, __shfl_xor_sync(kFull, mn.x, o));
     mn.y = fminf(mn.y, __shfl_xor_sync(kFull, mn.y, o));
     mn.z = fminf(mn.z, __shfl_xor_sync(kFull, mn.z, o));
@@ -541,7 +548,7 @@ __global__ void k_cull(Dev d, float rcull2) {
       c1 = c1 < d.capCand ? c1 : d.capCand;
       d.candStart[iBlock] = c0;
       int tiles[kWorkLevels], items[kWorkLevels];
-      const int L = work_split(c1 - c0, d.tilesPerWork, d.tailTiles, tiles, items);
+      const int L = work_split(c1 - c0, ri.tilesPerWork, ri.tailTiles, tiles, items);
       for (int l = 0; l < L; l++)
         if (items[l]) atomicAdd(&d.ctr->levelCount[l], items[l]);
     }
@@ -554,7 +561,8 @@ __global__ void k_cull(Dev d, float rcull2) {
   }
 }
 
-// 10/12. Exclusion rows of a candidate tile: one warp, lane = i atom.
+// 10/12. Exclusion word of one atom (lane of iBlock) against the 32 atoms of
+//        jBlock: bit b is clear where atom b is an excluded partner.
 __device__ __forceinline__ uint32_t excl_row(const Dev &d, int iBlock, int jBlock, int lane) {
   uint32_t row = 0xFFFFFFFFu;
   int a = d.slotAtom[32 * iBlock + lane];
@@ -637,7 +645,8 @@ __global__ void k_excl(Dev d) {
       const int v = lane < nb ? d.exclBlk[kExclBlk * t.w + lane] : -1;
       scan = __any_sync(kFull, v == t.x);
     }
-    uint32_t row = scan ? excl_row(d, t.w, t.x, lane) : 0xFFFFFFFFu;
+    // the word of j atom `lane` over the i atoms: it travels with the j atom
+    uint32_t row = scan ? excl_row(d, t.x, t.w, lane) : 0xFFFFFFFFu;
     bool any = __any_sync(kFull, row != 0xFFFFFFFFu);
     if (!kWrite) {
       if (lane == 0) d.candFlag[c] = any ? 1 : 0;
@@ -680,11 +689,12 @@ __global__ void k_work(Dev d) {
   const int lane = threadIdx.x & 31, nWarps = (gridDim.x * blockDim.x) >> 5;
   for (int b = t >> 5; b < B; b += nWarps) {
     const int c0 = d.candStart[b], nc = d.candStart[b + 1] - c0;
+    const RepInfo &ri = d.rep[d.blockRep[b]];
     int tiles[kWorkLevels], items[kWorkLevels];
-    const int L = work_split(nc, d.tilesPerWork, d.tailTiles, tiles, items);
+    const int L = work_split(nc, ri.tilesPerWork, ri.tailTiles, tiles, items);
     int s = c0;  // first candidate of the level (the order of work_walk)
     for (int l = 0; l < L; l++) {
-      const int size = work_item_size(d.tilesPerWork, l), end = s + tiles[l];
+      const int size = work_item_size(ri.tilesPerWork, l), end = s + tiles[l];
       if (items[l]) {
         int base = 0;
         if (lane == 0) base = off[l] + atomicAdd(&d.ctr->levelFill[l], items[l]);

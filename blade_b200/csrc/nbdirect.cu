@@ -10,18 +10,17 @@
 //    candidate, ballot), then walks the surviving tiles; the persistent warps
 //    pull items from a counter, longest first once a launch has measured
 //    their cycles (k_order).
-//  * Tiles without exclusion mask and MSLD atom are streamed: their j atoms
-//    that can reach the i block are queued per warp and evaluated in rounds
-//    in which each lane holds two i atoms and one j atom, the pair math of
-//    the two pairs in packed FP32x2 instructions, the j atom (coordinates,
-//    charge, LJ parameters, force) rotating through a group of lanes with
-//    __shfl_sync, so every j force returns to its lane without a butterfly
-//    reduction (the reference spends 15 xor-shuffles per j atom).
-//  * Masked and MSLD tiles are evaluated per tile: lane l owns i atom l and
-//    the compacted j atoms rotate through groups of 32, 16, 8 or 4 lanes.
+//  * The j atoms of the surviving tiles that can reach the i block are queued
+//    per warp in shared memory and evaluated in rounds of 32, whatever tile
+//    they come from: each lane holds four i atoms and meets one queued j atom
+//    per step, the pair math in packed FP32x2 instructions (eval_round); the j
+//    force rotates through a group of lanes with __shfl_sync, so it returns to
+//    its lane without a butterfly reduction (the reference spends 15
+//    xor-shuffles per j atom).  Exclusion masks travel with the j atom; MSLD
+//    pairs have a queue of their own.
 //  * Accumulation in int64 fixed point (2^-32 units): i forces once per work
-//    item, j forces once per queued atom or tile chunk, energy per pair and
-//    dU/dlambda per work item.  The FP32 partial sums inside a work item have
+//    item, j forces once per queued atom, energy per pair and dU/dlambda once
+//    per round.  The FP32 partial sums inside a work item have
 //    a fixed order, so results do not depend on which warp, CTA or launch
 //    runs which work item, nor on the order in which the items are taken.
 //  * Pair math in FP32: rsqrt, erfc as exp(-x^2)*P6(1/(1+p x)) sharing the
@@ -87,6 +86,27 @@ __device__ __forceinline__ float erfcx_poly(float t) {
 __device__ __forceinline__ long long to_fix(float v) {
   return __float2ll_rn(v * kFixScaleF);
 }
+
+// Sum of to_fix over a round's pairs (at most 32 a lane) without a 64-bit
+// conversion per pair: v = hi 2^-12 + lo 2^-32 with both parts rounded by adding
+// 1.5 2^23, whose low mantissa bits are then the integer.  hi is even in units
+// of 2^-32, so the rounding of lo is the rounding of v, and the sum is that of
+// to_fix bit for bit; |v| >= 1000 (and NaN) takes to_fix itself.
+struct FixSum {
+  int hi = 0, lo = 0;
+  __device__ __forceinline__ void add(float v, long long &sum) {
+    if (!(fabsf(v) < 1000.f)) {
+      sum += to_fix(v);
+      return;
+    }
+    constexpr float kMagic = 12582912.f;  // 1.5 2^23
+    const float th = fmaf(v, 4096.f, kMagic);
+    const float tl = fmaf(fmaf(v, 4096.f, -(th - kMagic)), 1048576.f, kMagic);
+    hi += __float_as_int(th) - __float_as_int(kMagic);
+    lo += __float_as_int(tl) - __float_as_int(kMagic);
+  }
+  __device__ __forceinline__ long long total() const { return (long long)hi * 1048576 + lo; }
+};
 
 __device__ __forceinline__ void red_add(long long *p, long long v) {
   atomicAdd(reinterpret_cast<unsigned long long *>(p), static_cast<unsigned long long>(v));
@@ -197,63 +217,16 @@ struct KArgs {
   int count;               // count in-cutoff pairs (energy variants only)
 };
 
-// One non-alchemical pair at r2 < rCut^2: returns (dE/dr)/r and, with
-// ENERGY, the pair energy.  PME + VFSWITCH (the production combination) is
-// written out with the switching algebra folded:
-//   VFSWITCH dE/dr * r = 6 c6 a r^-3 - 12 c12 b r^-6   (nbdirect.cu:336-346)
-// with a, b = (r^-3, r^-6) inside rSwitch and (k6 (r^-3 - rc^-3),
-// k12 (r^-6 - rc^-6)) outside; in combination mode this is
-// e6 w (a - w b) with w = Rmin^6 r^-3.  Other methods use pair_terms.
+// One pair at distance r = 1/rinv, r2 = r^2, of any method: returns (dE/dr)/r and
+// the pair energy.  PME + VFSWITCH, the production combination, is written out
+// below for two pairs at once.
 template <int ELEC, int VDW, bool ENERGY, bool COMBINE>
-__device__ __forceinline__ float plain_pair(const PairConst &pc, float r2, float qq, const float2 *sLJ,
-                                            int rowI, int tj, float2 ljI, float2 ljJ, float &E) {
-  const float rinv = rsqrt_approx(r2);
-  const float r = r2 * rinv;
-  if (ELEC == 1 && VDW == 0) {
-    const float t = rcp_approx(fmaf(pc.pBeta, r, 1.0f));
-    const float g = ex2_approx(pc.mBeta2Log2e * r2);
-    const float p = erfcx_poly(t);
-    const float qg = qq * g;
-    const float rinv2 = rinv * rinv;
-    const float rinv3 = rinv2 * rinv;
-    const float rinv6 = rinv3 * rinv3;
-    const bool in = r < pc.rswitch;
-    const float a = in ? rinv3 : fmaf(pc.k6, rinv3, -pc.k6rci3);
-    const float b = in ? rinv6 : fmaf(pc.k12, rinv6, -pc.k12rci6);
-    float flr, c12 = 0.f, c6 = 0.f;
-    if (COMBINE) {
-      const float e6 = ljI.x * ljJ.x;
-      const float R = ljI.y + ljJ.y;
-      const float R2 = R * R;
-      const float R6 = R2 * R2 * R2;
-      const float w = R6 * rinv3;
-      flr = e6 * w * fmaf(-w, b, a);
-      if (ENERGY) {
-        c6 = (e6 * (1.f / 6.f)) * R6;
-        c12 = (e6 * (1.f / 12.f)) * R6 * R6;
-      }
-    } else {  // the shared table holds (12 c12, 6 c6)
-      const float2 v = sLJ[rowI + tj];
-      flr = fmaf(v.y * a, rinv3, -(v.x * b) * rinv6);
-      if (ENERGY) {
-        c12 = v.x * (1.f / 12.f);
-        c6 = v.y * (1.f / 6.f);
-      }
-    }
-    if (ENERGY) {
-      const float pe = in ? fmaf(rinv6, rinv6, -pc.dv12) : b * (rinv6 - pc.rci6);
-      const float qe = in ? rinv6 - pc.dv6 : a * (rinv3 - pc.rci3);
-      E = qg * p * rinv + (c12 * pe - c6 * qe);
-    }
-    // Coulomb part of (dE/dr) r: -qq g (p / r + 2 beta / sqrt(pi))
-    return (flr - qg * fmaf(p, rinv, pc.twoBetaSqrtPi)) * rinv2;
-  } else {
-    float c12, c6;
-    lj_params<COMBINE>(sLJ, rowI, tj, ljI, ljJ, c12, c6);
-    float dEdr;
-    pair_terms<ELEC, VDW, ENERGY>(pc, r, r2, rinv, qq, c12, c6, dEdr, E);
-    return dEdr * rinv;
-  }
+__device__ __forceinline__ float general_pair(const PairConst &pc, float r2, float rinv, float r, float qq,
+                                              const float2 *sLJ, int rowI, int tj, float2 ljI, float2 ljJ, float &E) {
+  float c12, c6, dEdr;
+  lj_params<COMBINE>(sLJ, rowI, tj, ljI, ljJ, c12, c6);
+  pair_terms<ELEC, VDW, ENERGY>(pc, r, r2, rinv, qq, c12, c6, dEdr, E);
+  return dEdr * rinv;
 }
 
 // ---------------------------------------------------------------------------
@@ -263,22 +236,26 @@ __device__ __forceinline__ float plain_pair(const PairConst &pc, float r2, float
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 sel2(bool x, bool y, float2 a, float2 b) {
   return make_float2(x ? a.x : b.x, y ? a.y : b.y);
 }
 
-// Two PME + VFSWITCH pairs at squared distances r2 (.x for pair A, .y for B):
-// returns (dE/dr)/r for both; with ENERGY also their energies.  Same
-// algebra as plain_pair<PME, VFSWITCH>: erfc(beta r) = exp(-beta^2 r^2) P6(t),
-// VFSWITCH folded outside rSwitch.  Table mode takes (12 c12, 6 c6), combine
-// mode (e6, R) = (sqrt(12 eps_i) sqrt(12 eps_j), Rmin/2_i + Rmin/2_j).
+// Two PME + VFSWITCH pairs at distances r = 1/rinv, r2 = r^2 (one in .x, one in
+// .y): returns (dE/dr)/r for both; with ENERGY also their energies.
+//   erfc(beta r) = exp(-beta^2 r^2) P6(t),
+//   VFSWITCH dE/dr * r = 6 c6 a r^-3 - 12 c12 b r^-6   (nbdirect.cu:336-346)
+// with a, b = (r^-3, r^-6) inside rSwitch and (k6 (r^-3 - rc^-3),
+// k12 (r^-6 - rc^-6)) outside; k6, k12 > 1 and the two forms meet at rSwitch,
+// so a and b are the smaller of each.  In combination mode this is
+// e6 w (a - w b) with w = Rmin^6 r^-3.  Table mode takes (12 c12, 6 c6), combine
+// mode (e6, R) = (sqrt(12 eps_i) sqrt(12 eps_j), Rmin/2_i + Rmin/2_j).  nqq is
+// the negative charge product and nb = -b, so no sign costs an instruction.
 template <bool ENERGY, bool COMBINE>
-__device__ __forceinline__ float2 pme_vfsw_pair2(const PairConst &pc, float2 r2, float2 qq, float2 lj0, float2 lj1,
-                                                 float2 &E) {
-  const float2 rinv = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
-  const float2 r = mul2(r2, rinv);
+__device__ __forceinline__ float2 pme_vfsw_pair2(const PairConst &pc, float2 r2, float2 rinv,
+                                                 float2 r, float2 nqq, float2 lj0, float2 lj1, float2 &E) {
   const float2 targ = fma2(f2(pc.pBeta), r, f2(1.0f));
   const float2 t = make_float2(rcp_approx(targ.x), rcp_approx(targ.y));
   const float2 garg = mul2(f2(pc.mBeta2Log2e), r2);
@@ -290,290 +267,418 @@ __device__ __forceinline__ float2 pme_vfsw_pair2(const PairConst &pc, float2 r2,
   float2 po = fma2(f2(kErfcC5), t2, f2(kErfcC3));
   po = fma2(po, t2, f2(kErfcC1));
   const float2 p = fma2(po, t, pe);
-  const float2 qg = mul2(qq, g);
+  const float2 nqg = mul2(nqq, g);
   const float2 rinv2 = mul2(rinv, rinv);
   const float2 rinv3 = mul2(rinv2, rinv);
   const float2 rinv6 = mul2(rinv3, rinv3);
-  const bool inA = r.x < pc.rswitch, inB = r.y < pc.rswitch;
-  const float2 a = sel2(inA, inB, rinv3, fma2(f2(pc.k6), rinv3, f2(-pc.k6rci3)));
-  const float2 b = sel2(inA, inB, rinv6, fma2(f2(pc.k12), rinv6, f2(-pc.k12rci6)));
+  const float2 ao = fma2(f2(pc.k6), rinv3, f2(-pc.k6rci3));
+  const float2 nbo = fma2(f2(-pc.k12), rinv6, f2(pc.k12rci6));
+  const float2 a = make_float2(fminf(rinv3.x, ao.x), fminf(rinv3.y, ao.y));
+  const float2 nb = make_float2(fmaxf(-rinv6.x, nbo.x), fmaxf(-rinv6.y, nbo.y));
   float2 flr, c12, c6;
   if (COMBINE) {  // lj0 = e6, lj1 = R
     const float2 R2 = mul2(lj1, lj1);
     const float2 R6 = mul2(mul2(R2, R2), R2);
     const float2 w = mul2(R6, rinv3);
-    flr = mul2(mul2(lj0, w), fma2(mul2(w, f2(-1.f)), b, a));
+    flr = mul2(mul2(lj0, w), fma2(w, nb, a));
     if (ENERGY) {
       c6 = mul2(mul2(lj0, f2(1.f / 6.f)), R6);
       c12 = mul2(mul2(mul2(lj0, f2(1.f / 12.f)), R6), R6);
     }
   } else {        // lj0 = 12 c12, lj1 = 6 c6
-    flr = fma2(mul2(lj1, a), rinv3, mul2(mul2(mul2(lj0, f2(-1.f)), b), rinv6));
+    flr = fma2(mul2(lj1, a), rinv3, mul2(mul2(lj0, nb), rinv6));
     if (ENERGY) {
       c12 = mul2(lj0, f2(1.f / 12.f));
       c6 = mul2(lj1, f2(1.f / 6.f));
     }
   }
   if (ENERGY) {
+    const bool inA = r.x < pc.rswitch, inB = r.y < pc.rswitch;
     const float2 pe_in = fma2(rinv6, rinv6, f2(-pc.dv12));
-    const float2 pe_out = mul2(b, add2(rinv6, f2(-pc.rci6)));
-    const float2 qe_in = add2(rinv6, f2(-pc.dv6));
-    const float2 qe_out = mul2(a, add2(rinv3, f2(-pc.rci3)));
+    const float2 pe_out = mul2(nb, sub2(f2(pc.rci6), rinv6));
+    const float2 qe_in = sub2(f2(pc.dv6), rinv6);
+    const float2 qe_out = mul2(a, sub2(f2(pc.rci3), rinv3));
     const float2 pe2 = sel2(inA, inB, pe_in, pe_out);
-    const float2 qe2 = sel2(inA, inB, qe_in, qe_out);
-    E = fma2(mul2(qg, p), rinv, fma2(c12, pe2, mul2(mul2(c6, qe2), f2(-1.f))));
+    const float2 nqe2 = sel2(inA, inB, qe_in, qe_out);
+    E = fma2(c12, pe2, fma2(c6, nqe2, mul2(mul2(mul2(nqg, f2(-1.f)), p), rinv)));
   }
   // Coulomb part of (dE/dr) r: -qq g (p / r + 2 beta / sqrt(pi))
-  return mul2(fma2(mul2(qg, f2(-1.f)), fma2(p, rinv, f2(pc.twoBetaSqrtPi)), flr), rinv2);
+  return mul2(fma2(nqg, fma2(p, rinv, f2(pc.twoBetaSqrtPi)), flr), rinv2);
 }
 
-
-
-// Per-lane loads of one candidate tile (its j slot for this lane).
-template <int ALCH>
+// Per-lane loads of one candidate tile: the j slot of this lane.  Empty slots
+// hold a position far outside every cutoff (k_pack).
+template <bool COMBINE, int ALCH>
 struct TileFetch {
-  int jBlock, code, mIdx, atom, siteBlock;
+  int jBlock, code, t, siteBlock;
   float4 xj;
-  uint32_t row;
+  float2 lj;
+  uint32_t mask;  // i lanes this j atom may meet
   __device__ __forceinline__ void fetch(const Dev &d, int4 cand, int c, int lane) {
     jBlock = __shfl_sync(kFull, cand.x, c);
     code = __shfl_sync(kFull, cand.y, c);
-    mIdx = __shfl_sync(kFull, cand.z, c);
+    const int mIdx = __shfl_sync(kFull, cand.z, c);
     const int jslot = 32 * jBlock + lane;
     xj = d.xyzq[jslot];
-    atom = d.slotAtom[jslot];
+    if (COMBINE) lj = d.slotLj[jslot];
+    else t = d.slotType[jslot];
     siteBlock = ALCH ? d.slotSiteBlock[jslot] : 0;
-    row = mIdx >= 0 ? d.masks[32 * (size_t)mIdx + lane] : kFull;
+    mask = mIdx >= 0 ? d.masks[32 * (size_t)mIdx + lane] : kFull;
   }
 };
 
-// j-side registers that travel with the rotation.
-template <bool COMBINE, int ALCH>
-struct JRegs {
-  float x, y, z, q;
-  int meta;                // original j lane << 16 | LJ type (table) ; original lane (combine)
-  float ex, er;            // combine mode: sqrt(2 eps), Rmin/2
-  int b;                   // MSLD siteBlock
-  float l;                 // lambda of b
-  float fx, fy, fz, fl;
+// ---------------------------------------------------------------------------
+// Rounds.  The j atoms of a work item's tiles that can reach the i block are
+// queued per warp in shared memory with all that a pair needs of them (shifted
+// position and charge, LJ parameters, accumulator slot, the i lanes they may
+// meet), whatever tile they come from, and evaluated in rounds of up to 32.
+//
+// The i block is two halves of 16 atoms, lower and upper in z (its column is
+// sorted by z), each with an AABB of its own, and each half has its own queue:
+// a j atom that reaches one half only is not paired with the other.  The two
+// queues are interleaved, place p of the lower in .x and of the upper in .y.
+//
+// In a round lane l = 8 g + r holds four i atoms, r and r + 8 of either half, so
+// every group g of 8 lanes covers the block, and group g owns S of the 4 S
+// places (S = 8, 4, 2 or 1).  At step k the lane meets place (r + k) mod S of its
+// group: it reads the two entries from shared memory, meets the lower one with
+// its two lower atoms and the upper one with its two upper atoms as two packed
+// FP32x2 pairs, and hands the entries' force accumulators to the lane before
+// it, so after S steps every accumulator is back in its lane; groups of S lanes
+// of one group hold the same entries and are summed by xor shuffles, and each
+// entry's force is added to the fixed-point accumulators once.
+//
+// Bound by the issue of FP32 and the latencies inside a step.  A step of four
+// pairs issues 6 shared-memory loads, which depend on nothing and whose register
+// pairs are the packed operands as they are, and 6 shuffles; rounds that
+// rotated the j atom through shuffles against the whole block needed 18
+// shuffles in a chain and 1.2 (rCut 12 A) to 1.3 times (9 A) the steps.
+//
+// An entry whose mask is not full (an excluded partner, a tile against
+// itself) makes its round test the mask per pair; there are few of them.
+// MSLD pairs (ALCH) have queues of their own: every j atom of an i block with
+// MSLD atoms, and MSLD j atoms of other blocks.
+// ---------------------------------------------------------------------------
+// Places of a queue.  A round is due when both halves have 32 entries, or when
+// one half could overflow with the next tile, so the halves may differ by up to
+// PLACES - 64 entries before a round runs half empty.
+// Measured: 64 places 0.5-1 % slower than 96 without MSLD, 128 no faster; with
+// MSLD, 96 places leave too little L1 (batch of 32 small boxes 90 us against 76).
+template <int ALCH>
+constexpr int queue_places() {
+  return ALCH ? 64 : 96;
+}
 
-  // withAlch: also the MSLD fields (tiles without MSLD atoms never read them)
-  __device__ __forceinline__ void move(int src, int width, bool withMeta = true, bool withAlch = true) {
-    x = __shfl_sync(kFull, x, src, width);
-    y = __shfl_sync(kFull, y, src, width);
-    z = __shfl_sync(kFull, z, src, width);
-    q = __shfl_sync(kFull, q, src, width);
-    if (withMeta) meta = __shfl_sync(kFull, meta, src, width);
+template <bool COMBINE, bool MSLD, int PLACES>
+struct Queue {
+  static constexpr int kPlaces = PLACES;
+  // .x lower, .y upper half's entry; x, y, z negated, so that a difference is an addition
+  float2 x[PLACES], y[PLACES], z[PLACES], q[PLACES];
+  float2 e[COMBINE ? PLACES : 1], R[COMBINE ? PLACES : 1];  // sqrt(12 eps), Rmin/2
+  int2 t[COMBINE ? 1 : PLACES];                        // type index
+  int2 slot[PLACES];
+  uint2 mask[PLACES];
+  int2 b[MSLD ? PLACES : 1];      // siteBlock
+  float2 lam[MSLD ? PLACES : 1];  // its lambda
+};
+
+// One half's part of a place (an element of each array).
+__device__ __forceinline__ float &half_of(float2 &v, bool up) { return up ? v.y : v.x; }
+__device__ __forceinline__ int &half_of(int2 &v, bool up) { return up ? v.y : v.x; }
+__device__ __forceinline__ uint32_t &half_of(uint2 &v, bool up) { return up ? v.y : v.x; }
+
+// The four i atoms of a lane: [h].x atom r + 8 h, [h].y atom 16 + r + 8 h.
+struct IAtoms {
+  float2 x[2], y[2], z[2], nq[2];  // nq: negative scaled charge
+  float2 e6[2], R[2];  // combine mode: (sqrt(12 eps), Rmin/2)
+  int2 row[2];         // table mode: type * nTypes
+};
+
+// Sums over the groups of a warp a value per i atom (laid out as in IAtoms):
+// lane l receives the total of atom l.
+__device__ __forceinline__ float sum_groups(const float2 (&f)[2], int lane) {
+  const bool up = lane & 16, odd = lane & 8;
+  float k0 = up ? f[0].y : f[0].x, k1 = up ? f[1].y : f[1].x;
+  k0 += __shfl_xor_sync(kFull, up ? f[0].x : f[0].y, 16);
+  k1 += __shfl_xor_sync(kFull, up ? f[1].x : f[1].y, 16);
+  return (odd ? k1 : k0) + __shfl_xor_sync(kFull, odd ? k0 : k1, 8);
+}
+
+// MSLD scaling of one pair (nbdirect.cu:244-254).
+__device__ __forceinline__ bool same_site(int bi, int bj) { return ((bi ^ bj) & 0xFFFF0000) == 0; }
+__device__ __forceinline__ float msld_scale(int bi, int bj, float li, float lj) {
+  return same_site(bi, bj) ? (bi == bj ? lj : 0.f) : li * lj;
+}
+
+// KIND 0: no masks; 1: masks; 2: masks and MSLD scaling; 3: also soft core.
+template <int ELEC, int VDW, bool ENERGY, bool COMBINE, int KIND, class Q>
+__device__ __forceinline__ void eval_round(const Dev &d, const PairConst &pc, const float2 *sLJ, const Q &q, int head,
+                                           int CL, int CU, int S, int lane, int iBlock, const IAtoms &I,
+                                           const float *sLam, long long *sAccL, float2 (&fx)[2], float2 (&fy)[2],
+                                           float2 (&fz)[2], long long &ei, unsigned long long &pairs, int count) {
+  constexpr bool MSLD = KIND >= 2;
+  const int r = lane & 7, base = head + (lane >> 3) * S;
+  float2 jfx = f2(0.f), jfy = f2(0.f), jfz = f2(0.f), jfl = f2(0.f);
+  FixSum sum;
+  int2 bi[2];
+  float2 li[2], fl[2];
+  if (MSLD) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      bi[h].x = d.slotSiteBlock[32 * iBlock + r + 8 * h];
+      bi[h].y = d.slotSiteBlock[32 * iBlock + 16 + r + 8 * h];
+      li[h] = make_float2(bi[h].x ? sLam[bi[h].x & 0xFFFF] : 1.f, bi[h].y ? sLam[bi[h].y & 0xFFFF] : 1.f);
+      fl[h] = f2(0.f);
+    }
+  }
+  for (int k = 0; k < S; k++) {
+    const int e = base + ((r + k) & (S - 1));
+    const float2 xj = q.x[e], yj = q.y[e], zj = q.z[e], qj = q.q[e];
+    float2 ej = f2(0.f), Rj = f2(0.f);
+    int2 tj = make_int2(0, 0);
     if (COMBINE) {
-      ex = __shfl_sync(kFull, ex, src, width);
-      er = __shfl_sync(kFull, er, src, width);
+      ej = q.e[e];
+      Rj = q.R[e];
+    } else {
+      tj = q.t[e];
     }
-    if (ALCH && withAlch) {
-      b = __shfl_sync(kFull, b, src, width);
-      l = __shfl_sync(kFull, l, src, width);
+    uint2 m = make_uint2(0, 0);
+    if (KIND >= 1) {
+      m = q.mask[e];
+      m.x >>= r;
+      m.y >>= r;
     }
-  }
-  __device__ __forceinline__ void move_forces(int src, int width, bool alch) {
-    fx = __shfl_sync(kFull, fx, src, width);
-    fy = __shfl_sync(kFull, fy, src, width);
-    fz = __shfl_sync(kFull, fz, src, width);
-    if (ALCH && alch) fl = __shfl_sync(kFull, fl, src, width);
-  }
-};
-
-// gj rotation steps of a tile without MSLD scaling.  MASKED tiles test the
-// exclusion/diagonal row bit of the current j (its original lane travels in
-// J.meta); the others rely on far-away sentinels for empty slots.
-template <int ELEC, int VDW, bool ENERGY, bool COMBINE, bool MASKED, int ALCH>
-__device__ __forceinline__ void plain_loop(JRegs<COMBINE, ALCH> &J, const float4 &xi, uint32_t row, int gj,
-                                           int rot, const PairConst &pc, const float2 *sLJ, int rowI,
-                                           float2 ljI, float &fix, float &fiy, float &fiz, long long &ei,
-                                           unsigned long long &pairs, int count) {
-#pragma unroll 4
-  for (int k = 0; k < gj; k++) {
-    const float dx = xi.x - J.x, dy = xi.y - J.y, dz = xi.z - J.z;
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    bool act = r2 < pc.rc2;
-    if (MASKED) act = act && ((row >> (COMBINE ? J.meta : (J.meta >> 16))) & 1u);
-    if (!ENERGY) {
-      // Branch-free: the warp evaluates the pair math whenever any of its
-      // lanes is in range, so every lane computes it and lanes out of range
-      // (or excluded) select zero -- no divergent branch to enter and leave.
-      float E = 0.f;
-      float fs = plain_pair<ELEC, VDW, ENERGY, COMBINE>(pc, r2, xi.w * J.q, sLJ, rowI, J.meta & 0xFFFF, ljI,
-                                                        make_float2(J.ex, J.er), E);
-      fs = act ? fs : 0.f;
-      fix = fmaf(fs, dx, fix); fiy = fmaf(fs, dy, fiy); fiz = fmaf(fs, dz, fiz);
-      J.fx = fmaf(-fs, dx, J.fx); J.fy = fmaf(-fs, dy, J.fy); J.fz = fmaf(-fs, dz, J.fz);
-    } else if (act) {  // energy steps (1 in 10) keep the branch: fewer live registers
-      float E = 0.f;
-      const float fs = plain_pair<ELEC, VDW, ENERGY, COMBINE>(pc, r2, xi.w * J.q, sLJ, rowI, J.meta & 0xFFFF,
-                                                              ljI, make_float2(J.ex, J.er), E);
-      fix = fmaf(fs, dx, fix); fiy = fmaf(fs, dy, fiy); fiz = fmaf(fs, dz, fiz);
-      J.fx = fmaf(-fs, dx, J.fx); J.fy = fmaf(-fs, dy, J.fy); J.fz = fmaf(-fs, dz, J.fz);
-      ei += to_fix(E);  // energies in fixed point per pair: exact sums of the FP32 pair values
-      if (count) pairs++;
+    int2 bj = make_int2(0, 0);
+    float2 lamj = f2(1.f);
+    if (MSLD) {
+      bj = q.b[e];
+      lamj = q.lam[e];
     }
-    J.move(rot, gj, MASKED || !COMBINE, false);
-    J.move_forces(rot, gj, false);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Streamed tiles.  The compacted j atoms of a work item's tiles that need no
-// exclusion mask and no MSLD scaling are queued in shared memory as entries
-// (j slot | shift code << 27) and evaluated in rounds of up to 32.  For these
-// rounds lane l holds two i atoms of the block, A = l mod 16 and B = A + 16,
-// so each half of the warp covers the whole i block, and one queued j atom:
-// with rounds of width gw (16, 8 or 4) half h takes entries h gw .. h gw +
-// gw - 1, one per lane of each of its 16 / gw groups of gw lanes.  The j atom
-// meets its lane's two i atoms in packed FP32x2 instructions and rotates
-// through the group with its force accumulator, so a rotation step moves one
-// j atom for two pairs.  After gw steps the groups of a half are summed by
-// xor shuffles and group 0 adds each entry's force to the fixed-point
-// accumulators, one addition per queued j atom.  A round costs gw steps for
-// up to 2 gw entries, so a tile contributes exactly its compacted j atoms and
-// only the last round of a work item is padded.
-// ---------------------------------------------------------------------------
-template <bool COMBINE>
-__device__ __forceinline__ void stream_load(const Dev &d, int e, const float4 *shifts, float &x, float &y,
-                                            float &z, float &q, int &t, float &ex, float &er) {
-  if (e < 0) {  // padding: far outside rCut of every i atom
-    x = 1.0e18f; y = 0.f; z = 0.f; q = 0.f; t = 0; ex = 0.f; er = 0.f;
-    return;
-  }
-  const int js = e & 0x7FFFFFF;
-  const float4 sh = shifts[e >> 27];
-  const float4 xj = d.xyzq[js];
-  x = xj.x + sh.x;
-  y = xj.y + sh.y;
-  z = xj.z + sh.z;
-  q = xj.w;
-  t = d.slotType[js];
-  if (COMBINE) {
-    const float2 lj = d.ljType[t];
-    ex = lj.x;
-    er = lj.y;
-  }
-}
-
-// The two i atoms of a lane in the streamed rounds: position and scaled
-// charge of A (.x) and B (.y), LJ parameters (combine mode) or table rows.
-struct IPair {
-  float2 x, y, z, q;
-  float2 e6, R;   // combine mode: (sqrt(12 eps), Rmin/2) of A and B
-  int rowA, rowB; // table mode: type * nTypes of A and B
-};
-
-template <int ELEC, int VDW, bool ENERGY, bool COMBINE>
-__device__ __forceinline__ void stream_round(const Dev &d, const PairConst &pc, const float2 *sLJ, const int *sS,
-                                             int C, int lane, const IPair &I, const float4 *shifts,
-                                             float2 &fix2, float2 &fiy2, float2 &fiz2, long long &ei,
-                                             unsigned long long &pairs, int count) {
-  const int gw = C > 16 ? 16 : (C > 8 ? 8 : 4);
-  const int cl = lane & (gw - 1);
-  const int eIdx = (lane >> 4) * gw + cl;
-  const int e = eIdx < C ? sS[eIdx] : -1;
-  float jx, jy, jz, jq, jex = 0.f, jer = 0.f;
-  int tj;
-  stream_load<COMBINE>(d, e, shifts, jx, jy, jz, jq, tj, jex, jer);
-  float jfx = 0.f, jfy = 0.f, jfz = 0.f;
-#pragma unroll 2
-  for (int k = 0; k < gw; k++) {
-    // packed operations with the j value replicated into both halves
-    const float2 dx = fma2(f2(jx), f2(-1.f), I.x);
-    const float2 dy = fma2(f2(jy), f2(-1.f), I.y);
-    const float2 dz = fma2(f2(jz), f2(-1.f), I.z);
-    const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-    const bool actA = r2.x < pc.rc2, actB = r2.y < pc.rc2;
-    const float2 qq = mul2(I.q, f2(jq));
-    float2 fs, E = f2(0.f);
-    if (ELEC == 1 && VDW == 0) {
-      float2 lj0, lj1;
-      if (COMBINE) {
-        lj0 = mul2(I.e6, f2(jex));
-        lj1 = add2(I.R, f2(jer));
-      } else {
-        const float2 vA = sLJ[I.rowA + tj], vB = sLJ[I.rowB + tj];
-        lj0 = make_float2(vA.x, vB.x);
-        lj1 = make_float2(vA.y, vB.y);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const float2 dx = add2(I.x[h], xj), dy = add2(I.y[h], yj), dz = add2(I.z[h], zj);
+      const float2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+      bool actA = r2.x < pc.rc2, actB = r2.y < pc.rc2;
+      if (KIND >= 1) {
+        actA = actA && (m.x & (1u << (8 * h)));
+        actB = actB && (m.y & (1u << (8 * h)));
       }
-      fs = pme_vfsw_pair2<ENERGY, COMBINE>(pc, r2, qq, lj0, lj1, E);
-    } else {
-      fs.x = plain_pair<ELEC, VDW, ENERGY, COMBINE>(pc, r2.x, qq.x, sLJ, I.rowA, tj,
-                                                    make_float2(I.e6.x, I.R.x), make_float2(jex, jer), E.x);
-      fs.y = plain_pair<ELEC, VDW, ENERGY, COMBINE>(pc, r2.y, qq.y, sLJ, I.rowB, tj,
-                                                    make_float2(I.e6.y, I.R.y), make_float2(jex, jer), E.y);
+      const float2 nqq = mul2(I.nq[h], qj);
+      const float2 rinv = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
+      const float2 rr = mul2(r2, rinv);
+      float2 s, re = rr, re2 = r2, reinv = rinv, dredr, dredll;
+      if (MSLD) {
+        s = make_float2(msld_scale(bi[h].x, bj.x, li[h].x, lamj.x), msld_scale(bi[h].y, bj.y, li[h].y, lamj.y));
+        dredr = f2(1.f);
+        dredll = f2(0.f);
+        if (KIND == 3) {  // soft core, nbdirect.cu:257-275
+          const float2 rs = fma2(f2(-pc.softR), s, f2(pc.softR));
+          auto soften = [&](float r1, float rs1, float &re1, float &re21, float &reinv1, float &dr, float &dl) {
+            const float u = __fdividef(r1, rs1);
+            const float f = fmaf(u * u * u, fmaf(-0.5f, u, 1.f), 0.5f);
+            dr = (3.f - 2.f * u) * u * u;
+            dl = -pc.softR * (f - dr * u);
+            re1 = f * rs1;
+            reinv1 = rcp_approx(re1);
+            re21 = re1 * re1;
+          };
+          if ((bi[h].x | bj.x) != 0 && rr.x < rs.x) soften(rr.x, rs.x, re.x, re2.x, reinv.x, dredr.x, dredll.x);
+          if ((bi[h].y | bj.y) != 0 && rr.y < rs.y) soften(rr.y, rs.y, re.y, re2.y, reinv.y, dredr.y, dredll.y);
+        }
+      }
+      float2 fs, E = f2(0.f);
+      constexpr bool needE = ENERGY || MSLD;
+      if (ELEC == 1 && VDW == 0) {
+        float2 lj0, lj1;
+        if (COMBINE) {
+          lj0 = mul2(I.e6[h], ej);
+          lj1 = add2(I.R[h], Rj);
+        } else {
+          const float2 vA = sLJ[I.row[h].x + tj.x], vB = sLJ[I.row[h].y + tj.y];
+          lj0 = make_float2(vA.x, vB.x);
+          lj1 = make_float2(vA.y, vB.y);
+        }
+        fs = pme_vfsw_pair2<needE, COMBINE>(pc, re2, reinv, re, nqq, lj0, lj1, E);
+      } else {
+        fs.x = general_pair<ELEC, VDW, needE, COMBINE>(pc, re2.x, reinv.x, re.x, -nqq.x, sLJ, I.row[h].x, tj.x,
+                                                       make_float2(I.e6[h].x, I.R[h].x), make_float2(ej.x, Rj.x), E.x);
+        fs.y = general_pair<ELEC, VDW, needE, COMBINE>(pc, re2.y, reinv.y, re.y, -nqq.y, sLJ, I.row[h].y, tj.y,
+                                                       make_float2(I.e6[h].y, I.R[h].y), make_float2(ej.y, Rj.y), E.y);
+      }
+      if (MSLD) {
+        // fs = (dE/dr_eff) / r_eff; U = s E(r_eff(r, s)): dU/dr / r = s fs (r_eff / r) dr_eff/dr
+        const float2 de = mul2(mul2(fs, re), s);  // s dE/dr_eff
+        float2 dl = KIND == 3 ? fma2(de, dredll, E) : E;  // dU/ds
+        fs = KIND == 3 ? mul2(mul2(de, dredr), rinv) : mul2(fs, s);
+        E = mul2(E, s);
+        dl = sel2(actA, actB, dl, f2(0.f));
+        // dU/dlambda routing, nbdirect.cu:400-415 (block 0 is no variable)
+        const bool sA = same_site(bi[h].x, bj.x), sB = same_site(bi[h].y, bj.y);
+        fl[h].x += sA ? (bi[h].x == bj.x ? dl.x : 0.f) : lamj.x * dl.x;
+        fl[h].y += sB ? (bi[h].y == bj.y ? dl.y : 0.f) : lamj.y * dl.y;
+        jfl.x += sA ? 0.f : li[h].x * dl.x;
+        jfl.y += sB ? 0.f : li[h].y * dl.y;
+      }
+      // branch-free: lanes out of range (or excluded) select zero
+      fs = sel2(actA, actB, fs, f2(0.f));
+      fx[h] = fma2(fs, dx, fx[h]);
+      fy[h] = fma2(fs, dy, fy[h]);
+      fz[h] = fma2(fs, dz, fz[h]);
+      // the j atoms' forces with the sign of the i side, negated below
+      jfx = fma2(fs, dx, jfx);
+      jfy = fma2(fs, dy, jfy);
+      jfz = fma2(fs, dz, jfz);
+      if (ENERGY) {
+        // energies in fixed point per pair: exact sums of the FP32 pair values
+        sum.add(actA ? E.x : 0.f, ei);
+        sum.add(actB ? E.y : 0.f, ei);
+        if (count) pairs += (unsigned long long)actA + (unsigned long long)actB;
+      }
     }
-    fs = sel2(actA, actB, fs, f2(0.f));
-    fix2 = fma2(fs, dx, fix2);
-    fiy2 = fma2(fs, dy, fiy2);
-    fiz2 = fma2(fs, dz, fiz2);
-    // the j atom's force with the sign of the i side, negated below
-    jfx = fmaf(fs.x, dx.x, fmaf(fs.y, dx.y, jfx));
-    jfy = fmaf(fs.x, dy.x, fmaf(fs.y, dy.y, jfy));
-    jfz = fmaf(fs.x, dz.x, fmaf(fs.y, dz.y, jfz));
-    if (ENERGY) {
-      if (actA) ei += to_fix(E.x);
-      if (actB) ei += to_fix(E.y);
-      if (count) pairs += (unsigned long long)actA + (unsigned long long)actB;
-    }
-    jx = __shfl_sync(kFull, jx, lane + 1, gw);
-    jy = __shfl_sync(kFull, jy, lane + 1, gw);
-    jz = __shfl_sync(kFull, jz, lane + 1, gw);
-    jq = __shfl_sync(kFull, jq, lane + 1, gw);
-    if (COMBINE) {
-      jex = __shfl_sync(kFull, jex, lane + 1, gw);
-      jer = __shfl_sync(kFull, jer, lane + 1, gw);
-    } else {
-      tj = __shfl_sync(kFull, tj, lane + 1, gw);
-    }
-    jfx = __shfl_sync(kFull, jfx, lane + 1, gw);
-    jfy = __shfl_sync(kFull, jfy, lane + 1, gw);
-    jfz = __shfl_sync(kFull, jfz, lane + 1, gw);
+    auto pass = [&](float2 &v) {
+      v.x = __shfl_sync(kFull, v.x, lane + 1, S);
+      v.y = __shfl_sync(kFull, v.y, lane + 1, S);
+    };
+    pass(jfx);
+    pass(jfy);
+    pass(jfz);
+    if (MSLD) pass(jfl);
   }
-  // the groups of a half hold the same entries: sum them (not across halves)
-  for (int o = 8; o >= gw; o >>= 1) {
-    jfx += __shfl_xor_sync(kFull, jfx, o);
-    jfy += __shfl_xor_sync(kFull, jfy, o);
-    jfz += __shfl_xor_sync(kFull, jfz, o);
+  if (ENERGY) ei += sum.total();
+  for (int o = 4; o >= S; o >>= 1) {
+    auto fold = [&](float2 &v) {
+      v.x += __shfl_xor_sync(kFull, v.x, o);
+      v.y += __shfl_xor_sync(kFull, v.y, o);
+    };
+    fold(jfx);
+    fold(jfy);
+    fold(jfz);
+    if (MSLD) fold(jfl);
   }
-  if ((lane & 15) < gw && e >= 0 && (jfx != 0.f || jfy != 0.f || jfz != 0.f)) {
-    const int S = 32 * d.maxBlocks;
-    const int js = e & 0x7FFFFFF;
-    red_add(&d.accF[js], to_fix(-jfx));
-    red_add(&d.accF[S + js], to_fix(-jfy));
-    red_add(&d.accF[2 * S + js], to_fix(-jfz));
-    if (!(isfinite(jfx) && isfinite(jfy) && isfinite(jfz))) atomicOr(&d.ctr->status, kStatusNonFinite);
+  const int place = base - head + r;
+  if (r < S) {
+    const int NS = 32 * d.maxBlocks;
+    const int2 js = q.slot[base + r];
+    auto deliver = [&](int j, float x, float y, float z) {
+      if (x == 0.f && y == 0.f && z == 0.f) return;
+      red_add(&d.accF[j], to_fix(-x));
+      red_add(&d.accF[NS + j], to_fix(-y));
+      red_add(&d.accF[2 * NS + j], to_fix(-z));
+      if (!(isfinite(x) && isfinite(y) && isfinite(z))) atomicOr(&d.ctr->status, kStatusNonFinite);
+    };
+    if (place < CL) deliver(js.x, jfx.x, jfy.x, jfz.x);
+    if (place < CU) deliver(js.y, jfx.y, jfy.y, jfz.y);
+    if (MSLD) {
+      const int2 b = q.b[base + r];
+      if (place < CL && jfl.x != 0.f && b.x)
+        atomicAdd(reinterpret_cast<unsigned long long *>(&sAccL[b.x & 0xFFFF]),
+                  static_cast<unsigned long long>(to_fix(jfl.x)));
+      if (place < CU && jfl.y != 0.f && b.y)
+        atomicAdd(reinterpret_cast<unsigned long long *>(&sAccL[b.y & 0xFFFF]),
+                  static_cast<unsigned long long>(to_fix(jfl.y)));
+    }
+  }
+  if (MSLD) {  // the block's dU/dlambda of this round
+    const float v = sum_groups(fl, lane);  // lane l: i atom l
+    const int b = d.slotSiteBlock[32 * iBlock + lane];
+    if (b && v != 0.f)
+      atomicAdd(reinterpret_cast<unsigned long long *>(&sAccL[b & 0xFFFF]),
+                static_cast<unsigned long long>(to_fix(v)));
   }
 }
+
+// A queue's fill: entries of the lower and upper half from place `head` on.
+template <int PLACES>
+struct Fill {
+  int nL = 0, nU = 0, head = 0;
+  __device__ __forceinline__ bool due(bool last) const {
+    const int most = nL > nU ? nL : nU, least = nL < nU ? nL : nU;
+    return least >= 32 || most > PLACES - 32 || (last && most > 0);
+  }
+  __device__ __forceinline__ int place(int n) const {
+    const int p = head + n;
+    return p >= PLACES ? p - PLACES : p;
+  }
+};
+
+// One round of a queue (places without an entry are padded with one far
+// outside every cutoff).
+template <int ELEC, int VDW, bool ENERGY, bool COMBINE, int ALCHQ, class Q>
+__device__ __forceinline__ void run_round(const Dev &d, const PairConst &pc, const float2 *sLJ, Q &q, Fill<Q::kPlaces> &f, int lane,
+                                          int iBlock, const IAtoms &I, const float *sLam, long long *sAccL,
+                                          float2 (&fx)[2], float2 (&fy)[2], float2 (&fz)[2], long long &ei,
+                                          unsigned long long &pairs, int count) {
+  // 32, 16, 8 or 4 places, whichever pads least: 20 left over go as 16 + 4
+  const int n = f.nL > f.nU ? f.nL : f.nU;
+  const int cap = n > 24 ? 32 : (n > 12 ? 16 : (n > 4 ? 8 : 4));
+  const int CL = f.nL < cap ? f.nL : cap, CU = f.nU < cap ? f.nU : cap;
+  const int at = f.head + lane;
+  if (lane < cap) {
+#pragma unroll
+    for (int up = 0; up < 2; up++)
+      if (lane >= (up ? CU : CL)) {
+        half_of(q.x[at], up) = -1.0e18f;
+        half_of(q.y[at], up) = half_of(q.z[at], up) = half_of(q.q[at], up) = 0.f;
+        if constexpr (COMBINE) half_of(q.e[at], up) = half_of(q.R[at], up) = 0.f;
+        else half_of(q.t[at], up) = 0;
+        half_of(q.mask[at], up) = 0xFFFFu;
+        if constexpr (ALCHQ != 0) {
+          half_of(q.b[at], up) = 0;
+          half_of(q.lam[at], up) = 1.f;
+        }
+      }
+  }
+  __syncwarp();
+  bool masked = false;
+  if (ALCHQ == 0) {
+    if (lane < cap) {
+      const uint2 m = q.mask[at];
+      masked = (m.x & m.y) != 0xFFFFu;
+    }
+    masked = __any_sync(kFull, masked);
+  }
+  if (ALCHQ != 0)
+    eval_round<ELEC, VDW, ENERGY, COMBINE, ALCHQ ? ALCHQ + 1 : 1>(d, pc, sLJ, q, f.head, CL, CU, cap >> 2, lane, iBlock,
+                                                                  I, sLam, sAccL, fx, fy, fz, ei, pairs, count);
+  else if (masked)
+    eval_round<ELEC, VDW, ENERGY, COMBINE, 1>(d, pc, sLJ, q, f.head, CL, CU, cap >> 2, lane, iBlock, I, sLam, sAccL, fx,
+                                              fy, fz, ei, pairs, count);
+  else
+    eval_round<ELEC, VDW, ENERGY, COMBINE, 0>(d, pc, sLJ, q, f.head, CL, CU, cap >> 2, lane, iBlock, I, sLam, sAccL, fx,
+                                              fy, fz, ei, pairs, count);
+  __syncwarp();  // the entries are read; their places may be refilled
+  f.head = f.place(cap);
+  f.nL -= CL;
+  f.nU -= CU;
+}
+
+// Per-warp shared memory of k_pair.
+template <bool COMBINE, int ALCH>
+struct WarpSmem {
+  Queue<COMBINE, false, queue_places<ALCH>()> plain;
+  Queue<COMBINE, true, queue_places<ALCH>()> msld;
+};
+template <bool COMBINE>
+struct WarpSmem<COMBINE, 0> {
+  Queue<COMBINE, false, queue_places<0>()> plain;
+};
 
 // ---------------------------------------------------------------------------
 // The pair kernel.
 // ALCH: 0 none, 1 MSLD scaling, 2 MSLD scaling + soft core.
-//
-// Tile processing with j compaction: the nj j atoms of a tile that lie within
-// rCut of the i block's AABB are taken in chunks of gj = 32, 16, 8 or 4
-// (every chunk but the last full), each replicated in groups of gj lanes.
-// Every lane keeps its own i atom and rotates through the gj j atoms of its
-// group, so a tile costs nj rounded up to a multiple of 4 steps instead of
-// 32; the group partial j forces are summed with xor shuffles and returned to
-// the owner lanes, one chunk per j atom.
 // ---------------------------------------------------------------------------
 template <int ELEC, int VDW, int ALCH, bool ENERGY, bool COMBINE>
 __global__ void __launch_bounds__(256, 2) k_pair(KArgs A) {
   pdl_wait();
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int sIdx[8][32];
-  __shared__ int sStream[8][128];  // queued entries of streamed tiles, per warp
   const Dev &d = A.d;
   const PairConst &pc = A.pc;
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
   const int nT = d.nTypes;
-  float2 *sLJ = reinterpret_cast<float2 *>(smem);
-  size_t off = COMBINE ? 0 : sizeof(float2) * nT * nT;
-  off = (off + 15) & ~size_t(15);
+  using Warp = WarpSmem<COMBINE, ALCH>;
+  Warp &ws = reinterpret_cast<Warp *>(smem)[threadIdx.x >> 5];
+  float2 *sLJ = reinterpret_cast<float2 *>(smem + 8 * sizeof(Warp));
+  const size_t off = 8 * sizeof(Warp) + (COMBINE ? 0 : (sizeof(float2) * nT * nT + 15) & ~size_t(15));
   long long *sAccL = reinterpret_cast<long long *>(smem + off);
   float *sLam = reinterpret_cast<float *>(smem + off + (ALCH ? sizeof(long long) * d.lamTotal : 0));
 
@@ -591,7 +696,7 @@ __global__ void __launch_bounds__(256, 2) k_pair(KArgs A) {
 
   const int status = d.ctr->status;
   const int nWork = (status & kStatusListInvalid) ? 0 : d.ctr->workCount;
-  const int S = 32 * d.maxBlocks;
+  const int NS = 32 * d.maxBlocks;
   unsigned long long pairs = 0;
 
   // after the first launch of a list the items are taken longest first, in
@@ -608,18 +713,15 @@ __global__ void __launch_bounds__(256, 2) k_pair(KArgs A) {
     const int c0 = wk.y;
     int c1 = d.candStart[iBlock + 1];
     c1 = c1 < c0 + (wk.x >> 22) ? c1 : c0 + (wk.x >> 22);
-    const int islot = 32 * iBlock + lane;
-    float4 xi = d.xyzq[islot];
-    const bool iValid = d.slotAtom[islot] >= 0;
-    if (!iValid) xi.x = -1.0e18f;  // empty i slot: never within rCut of any j
-    const int ti = d.slotType[islot];
-    const int rowI = ti * nT;
-    const float2 ljI = COMBINE ? d.ljType[ti] : make_float2(0.f, 0.f);
-    const int bi = ALCH ? d.slotSiteBlock[islot] : 0;
-    const float li = (ALCH && bi) ? sLam[bi & 0xFFFF] : 1.f;
     const RepInfo &ri = d.rep[d.blockRep[iBlock]];
     const float4 *shifts = ri.shift;  // image shift vectors by shift code
     const float4 imin = d.bmin[iBlock], imax = d.bmax[iBlock];
+    float4 hmin[2], hmax[2];  // the halves' boxes
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      hmin[u] = d.hmin[2 * iBlock + u];
+      hmax[u] = d.hmax[2 * iBlock + u];
+    }
 
     // per-step recull of this work item's candidates (recull.cu:41-122)
     int4 cand = make_int4(0, 0, -1, 0);
@@ -632,238 +734,114 @@ __global__ void __launch_bounds__(256, 2) k_pair(KArgs A) {
     }
     unsigned act = __ballot_sync(kFull, hit);
 
-    float fix = 0.f, fiy = 0.f, fiz = 0.f, fli = 0.f;
-    // i atoms A = lane mod 16 and B = A + 16 of the streamed rounds, their forces
-    IPair ip;
+    IAtoms I;
+    bool anyI = false;  // the i block holds MSLD atoms
     {
-      const int a = lane & 15;
-      ip.x = make_float2(__shfl_sync(kFull, xi.x, a), __shfl_sync(kFull, xi.x, a + 16));
-      ip.y = make_float2(__shfl_sync(kFull, xi.y, a), __shfl_sync(kFull, xi.y, a + 16));
-      ip.z = make_float2(__shfl_sync(kFull, xi.z, a), __shfl_sync(kFull, xi.z, a + 16));
-      ip.q = make_float2(__shfl_sync(kFull, xi.w, a), __shfl_sync(kFull, xi.w, a + 16));
-      if (COMBINE) {
-        ip.e6 = make_float2(__shfl_sync(kFull, ljI.x, a), __shfl_sync(kFull, ljI.x, a + 16));
-        ip.R = make_float2(__shfl_sync(kFull, ljI.y, a), __shfl_sync(kFull, ljI.y, a + 16));
-        ip.rowA = ip.rowB = 0;
-      } else {
-        ip.e6 = ip.R = f2(0.f);
-        ip.rowA = __shfl_sync(kFull, rowI, a);
-        ip.rowB = __shfl_sync(kFull, rowI, a + 16);
-      }
-    }
-    float2 fix2 = f2(0.f), fiy2 = f2(0.f), fiz2 = f2(0.f);
-    int nS = 0;        // entries queued in sStream[warp]
-    long long ei = 0;  // fixed-point energy of this lane's pairs
-    // The loads of each tile are issued one tile ahead, so their latency
-    // overlaps the compaction and chunk work of the tile before.
-    TileFetch<ALCH> nxt;
-    if (act) nxt.fetch(d, cand, __ffs(act) - 1, lane);
-    while (act) {
-      act &= act - 1;
-      const TileFetch<ALCH> cur = nxt;
-      if (act) nxt.fetch(d, cand, __ffs(act) - 1, lane);
-      const int jBlock = cur.jBlock;
-      const int code = cur.code;
-      const int mIdx = cur.mIdx;
-      const float4 sv = shifts[code];
-      const float shx = sv.x, shy = sv.y, shz = sv.z;
-      const int jslot = 32 * jBlock + lane;
-      const float jx = cur.xj.x + shx, jy = cur.xj.y + shy, jz = cur.xj.z + shz;
-      const int bj0 = ALCH ? cur.siteBlock : 0;
-      const bool jValid = cur.atom >= 0;
-      uint32_t row = cur.row;
-      if (jBlock == iBlock && code == 0) row &= (lane == 31) ? 0u : (kFull << (lane + 1));
-      if (!iValid) row = 0u;
-
-      // j atoms that can reach the i block (per-atom AABB test, nbdirect.cu:211)
-      float g, gap2;
-      g = fmaxf(fmaxf(imin.x - jx, jx - imax.x), 0.f);
-      gap2 = g * g;
-      g = fmaxf(fmaxf(imin.y - jy, jy - imax.y), 0.f);
-      gap2 = fmaf(g, g, gap2);
-      g = fmaxf(fmaxf(imin.z - jz, jz - imax.z), 0.f);
-      gap2 = fmaf(g, g, gap2);
-      const bool jin = jValid && gap2 < pc.rc2;
-      const unsigned jm = __ballot_sync(kFull, jin);
-      const int nj = __popc(jm);
-      if (nj == 0) continue;
-      const bool alchTile = ALCH ? __any_sync(kFull, (bi | bj0) != 0) : false;
-      // Tiles without an exclusion mask and off the diagonal need no per-step
-      // mask test: empty j slots and invalid i lanes sit far outside rCut.
-      const bool masked = mIdx >= 0 || (jBlock == iBlock && code == 0);
-
-      const int rank = __popc(jm & ((1u << lane) - 1u));
-      if (!masked && !alchTile) {  // streamed: queue the compacted j atoms, evaluate full chunks of 64
-        if (jin) sStream[warp][nS + rank] = jslot | (code << 27);
-        nS += nj;
-        __syncwarp();
-        if (nS >= 32) {
-          stream_round<ELEC, VDW, ENERGY, COMBINE>(d, pc, sLJ, sStream[warp], 32, lane, ip, shifts, fix2, fiy2,
-                                                   fiz2, ei, pairs, A.count);
-          const int rest = nS - 32;  // < 32
-          const int carry = lane < rest ? sStream[warp][32 + lane] : 0;
-          __syncwarp();
-          if (lane < rest) sStream[warp][lane] = carry;
-          __syncwarp();
-          nS = rest;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int h = k & 1, up = k >> 1, is = 32 * iBlock + (lane & 7) + 8 * k;
+        float4 xi = d.xyzq[is];
+        if (xi.x > 1.0e17f) xi.x = -1.0e18f;  // empty i slot: never within rCut of any j, nor of padding
+        half_of(I.x[h], up) = xi.x;
+        half_of(I.y[h], up) = xi.y;
+        half_of(I.z[h], up) = xi.z;
+        half_of(I.nq[h], up) = -xi.w;
+        if (COMBINE) {
+          const float2 lj = d.slotLj[is];
+          half_of(I.e6[h], up) = lj.x;
+          half_of(I.R[h], up) = lj.y;
+          half_of(I.row[h], up) = 0;
+        } else {
+          half_of(I.e6[h], up) = half_of(I.R[h], up) = 0.f;
+          half_of(I.row[h], up) = d.slotType[is] * nT;
         }
+      }
+      if (ALCH) anyI = __any_sync(kFull, d.slotSiteBlock[32 * iBlock + lane] != 0);
+    }
+    float2 fx[2], fy[2], fz[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) fx[h] = fy[h] = fz[h] = f2(0.f);
+    long long ei = 0;  // fixed-point energy of this lane's pairs
+    Fill<queue_places<ALCH>()> plain, msld;
+
+    // The loads of each tile are issued one tile ahead, so their latency
+    // overlaps the rounds and the queueing of the tile before.
+    TileFetch<COMBINE, ALCH> nxt;
+    if (act) nxt.fetch(d, cand, __ffs(act) - 1, lane);
+    while (true) {
+      if (plain.due(!act)) {
+        run_round<ELEC, VDW, ENERGY, COMBINE, 0>(d, pc, sLJ, ws.plain, plain, lane, iBlock, I, sLam, sAccL, fx, fy, fz,
+                                                 ei, pairs, A.count);
         continue;
       }
-      // compaction order: the p-th surviving j atom is lane sIdx[p]
-      if (jin) sIdx[warp][rank] = lane;
-      __syncwarp();
-      // j force of this lane's own j atom, delivered by the chunk that held it
-      float ofx = 0.f, ofy = 0.f, ofz = 0.f, ofl = 0.f;
-      // The nj surviving j atoms are processed in chunks of 32, 16, 8 or 4
-      // (32 only when more than 28 survive; otherwise 16 while more than 12
-      // remain, then 8, then 4), each replicated in groups of gj lanes, so a
-      // tile costs nj rounded up to a multiple of 4 rotation steps.
-      for (int done = 0; done < nj;) {
-        const int rem = nj - done;
-        const int gj = rem > 28 ? 32 : (rem > 12 ? 16 : (rem > 4 ? 8 : 4));
-        const int cnt = rem < gj ? rem : gj;
-        const int cl = lane & (gj - 1);
-        const int src = cl < cnt ? sIdx[warp][done + cl] : lane;
-        JRegs<COMBINE, ALCH> J;
-        {
-          const int js = 32 * jBlock + src;
-          const float4 xj = d.xyzq[js];
-          J.x = xj.x + shx;
-          J.y = xj.y + shy;
-          J.z = xj.z + shz;
-          J.q = xj.w;
-          const int tj = d.slotType[js];
-          J.meta = COMBINE ? src : ((src << 16) | tj);
-          if (COMBINE) {
-            const float2 lj2 = d.ljType[tj];
-            J.ex = lj2.x;
-            J.er = lj2.y;
-          }
-          if (ALCH && alchTile) {
-            J.b = d.slotSiteBlock[js];
-            J.l = J.b ? sLam[J.b & 0xFFFF] : 1.f;
-          }
+      if constexpr (ALCH != 0) {
+        if (msld.due(!act)) {
+          run_round<ELEC, VDW, ENERGY, COMBINE, ALCH>(d, pc, sLJ, ws.msld, msld, lane, iBlock, I, sLam, sAccL, fx, fy,
+                                                      fz, ei, pairs, A.count);
+          continue;
         }
-        if (cl >= cnt) J.x = 1.0e18f;  // empty compacted slot: never within rCut
-        J.fx = J.fy = J.fz = J.fl = 0.f;
-        const int rot = lane + 1;
+      }
+      if (!act) break;
+      act &= act - 1;
+      const TileFetch<COMBINE, ALCH> cur = nxt;
+      if (act) nxt.fetch(d, cand, __ffs(act) - 1, lane);
+      const float4 sv = shifts[cur.code];
+      const float4 xj = make_float4(cur.xj.x + sv.x, cur.xj.y + sv.y, cur.xj.z + sv.z, cur.xj.w);
+      uint32_t mask = cur.mask;
+      if (cur.jBlock == iBlock && cur.code == 0) mask &= (1u << lane) - 1u;  // each pair of the block once: i < j
 
-        if (!alchTile) {
-          if (masked)
-            plain_loop<ELEC, VDW, ENERGY, COMBINE, true>(J, xi, row, gj, rot, pc, sLJ, rowI, ljI, fix, fiy, fiz,
-                                                         ei, pairs, A.count);
-          else
-            plain_loop<ELEC, VDW, ENERGY, COMBINE, false>(J, xi, row, gj, rot, pc, sLJ, rowI, ljI, fix, fiy,
-                                                          fiz, ei, pairs, A.count);
-        } else if (ALCH) {
-          for (int k = 0; k < gj; k++) {
-            const float dx = xi.x - J.x, dy = xi.y - J.y, dz = xi.z - J.z;
-            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            const int jb = COMBINE ? J.meta : (J.meta >> 16);
-            if (((row >> jb) & 1u) && r2 < pc.rc2) {
-              float c12, c6;
-              lj_params<COMBINE>(sLJ, rowI, J.meta & 0xFFFF, ljI, make_float2(J.ex, J.er), c12, c6);
-              const float rinv = rsqrt_approx(r2);
-              const float r = r2 * rinv;
-              const int bj = J.b;
-              const float lj = J.l;
-              // MSLD scaling, nbdirect.cu:244-254
-              const bool sameSite = (bi & 0xFFFF0000) == (bj & 0xFFFF0000);
-              const float s = sameSite ? (bi == bj ? li : 0.f) : li * lj;
-              const bool pert = (bi | bj) != 0;
-              float rEff = r, rinvE = rinv, r2E = r2, dredr = 1.f, dredll = 0.f;
-              if (ALCH == 2 && pert) {  // soft core, nbdirect.cu:257-275
-                const float rSoft = pc.softR * (1.f - s);
-                if (r < rSoft) {
-                  const float q = __fdividef(r, rSoft);
-                  const float f = fmaf(q * q * q, fmaf(-0.5f, q, 1.f), 0.5f);
-                  dredr = (3.f - 2.f * q) * q * q;
-                  dredll = -pc.softR * (f - dredr * q);
-                  rEff = f * rSoft;
-                  rinvE = rcp_approx(rEff);
-                  r2E = rEff * rEff;
-                }
-              }
-              float dEdr, E;
-              pair_terms<ELEC, VDW, true>(pc, rEff, r2E, rinvE, xi.w * J.q, c12, c6, dEdr, E);
-              dEdr *= s;
-              if (pert) {  // dU/dlambda routing, nbdirect.cu:400-415
-                const float fl = fmaf(dEdr, dredll, E);
-                if (sameSite) {
-                  if (bi == bj) fli += fl;
-                } else {
-                  fli = fmaf(lj, fl, fli);
-                  J.fl = fmaf(li, fl, J.fl);
-                }
-              }
-              const float fs = dEdr * dredr * rinv;
-              fix = fmaf(fs, dx, fix); fiy = fmaf(fs, dy, fiy); fiz = fmaf(fs, dz, fiz);
-              J.fx = fmaf(-fs, dx, J.fx); J.fy = fmaf(-fs, dy, J.fy); J.fz = fmaf(-fs, dz, J.fz);
-              if (ENERGY) ei += to_fix(s * E);
-              if (ENERGY && A.count) pairs++;
-            }
-            J.move(rot, gj);
-            J.move_forces(rot, gj, true);
+      const bool toM = ALCH && (anyI || cur.siteBlock != 0);
+      const unsigned before = (1u << lane) - 1u;
+      // per half: j atoms that can reach it (per-atom AABB test, nbdirect.cu:211)
+#pragma unroll
+      for (int up = 0; up < 2; up++) {
+        float g, gap2;
+        g = fmaxf(fmaxf(hmin[up].x - xj.x, xj.x - hmax[up].x), 0.f);
+        gap2 = g * g;
+        g = fmaxf(fmaxf(hmin[up].y - xj.y, xj.y - hmax[up].y), 0.f);
+        gap2 = fmaf(g, g, gap2);
+        g = fmaxf(fmaxf(hmin[up].z - xj.z, xj.z - hmax[up].z), 0.f);
+        gap2 = fmaf(g, g, gap2);
+        const uint32_t mh = up ? mask >> 16 : mask & 0xFFFFu;
+        const bool jin = gap2 < pc.rc2 && mh != 0u;
+        auto put = [&](auto &q, int at) {
+          half_of(q.x[at], up) = -xj.x;
+          half_of(q.y[at], up) = -xj.y;
+          half_of(q.z[at], up) = -xj.z;
+          half_of(q.q[at], up) = xj.w;
+          if constexpr (COMBINE) {
+            half_of(q.e[at], up) = cur.lj.x;
+            half_of(q.R[at], up) = cur.lj.y;
+          } else {
+            half_of(q.t[at], up) = cur.t;
           }
+          half_of(q.slot[at], up) = 32 * cur.jBlock + lane;
+          half_of(q.mask[at], up) = mh;
+        };
+        const unsigned mp = __ballot_sync(kFull, jin && !toM);
+        if (jin && !toM) put(ws.plain, plain.place((up ? plain.nU : plain.nL) + __popc(mp & before)));
+        (up ? plain.nU : plain.nL) += __popc(mp);
+        if constexpr (ALCH != 0) {
+          const unsigned mm = __ballot_sync(kFull, jin && toM);
+          if (jin && toM) {
+            const int at = msld.place((up ? msld.nU : msld.nL) + __popc(mm & before));
+            put(ws.msld, at);
+            half_of(ws.msld.b[at], up) = cur.siteBlock;
+            half_of(ws.msld.lam[at], up) = cur.siteBlock ? sLam[cur.siteBlock & 0xFFFF] : 1.f;
+          }
+          (up ? msld.nU : msld.nL) += __popc(mm);
         }
-        // sum the group partials; group 0 lane p now holds compacted j done+p
-        float fx = J.fx, fy = J.fy, fz = J.fz, fl = J.fl;
-        for (int o = 16; o >= gj; o >>= 1) {
-          fx += __shfl_xor_sync(kFull, fx, o);
-          fy += __shfl_xor_sync(kFull, fy, o);
-          fz += __shfl_xor_sync(kFull, fz, o);
-          if (ALCH && alchTile) fl += __shfl_xor_sync(kFull, fl, o);
-        }
-        // deliver to the owner lane of each j atom of this chunk
-        const int from = (rank - done) & 31;
-        fx = __shfl_sync(kFull, fx, from);
-        fy = __shfl_sync(kFull, fy, from);
-        fz = __shfl_sync(kFull, fz, from);
-        if (ALCH && alchTile) fl = __shfl_sync(kFull, fl, from);
-        if (rank >= done && rank < done + cnt) {
-          ofx = fx; ofy = fy; ofz = fz; ofl = fl;
-        }
-        done += cnt;
       }
-      __syncwarp();  // sIdx is rewritten by the next tile
-      if (jin && (ofx != 0.f || ofy != 0.f || ofz != 0.f)) {
-        red_add(&d.accF[jslot], to_fix(ofx));
-        red_add(&d.accF[S + jslot], to_fix(ofy));
-        red_add(&d.accF[2 * S + jslot], to_fix(ofz));
-        if (!(isfinite(ofx) && isfinite(ofy) && isfinite(ofz))) atomicOr(&d.ctr->status, kStatusNonFinite);
-      }
-      if (ALCH && alchTile && jin && bj0 && ofl != 0.f)
-        atomicAdd(reinterpret_cast<unsigned long long *>(&sAccL[bj0 & 0xFFFF]),
-                  static_cast<unsigned long long>(to_fix(ofl)));
     }
-    // the rest of the queue (< 32 entries) in rounds of 32, 16 or 8 entries,
-    // whichever pads least: e.g. 20 entries as 16 + 8 (12 steps, not 16)
-    for (int off = 0; off < nS;) {
-      const int rem = nS - off;
-      const int cap = rem > 24 ? 32 : (rem > 12 ? 16 : 8);
-      const int cnt = rem < cap ? rem : cap;
-      stream_round<ELEC, VDW, ENERGY, COMBINE>(d, pc, sLJ, sStream[warp] + off, cnt, lane, ip, shifts, fix2, fiy2,
-                                               fiz2, ei, pairs, A.count);
-      off += cnt;
-    }
-    __syncwarp();  // sStream is rewritten by the next work item
-    // the two halves hold the same i atoms: after the sum, lane l < 16 has
-    // atom l in .x and lane l >= 16 atom l in .y
-    fix2.x += __shfl_xor_sync(kFull, fix2.x, 16); fix2.y += __shfl_xor_sync(kFull, fix2.y, 16);
-    fiy2.x += __shfl_xor_sync(kFull, fiy2.x, 16); fiy2.y += __shfl_xor_sync(kFull, fiy2.y, 16);
-    fiz2.x += __shfl_xor_sync(kFull, fiz2.x, 16); fiz2.y += __shfl_xor_sync(kFull, fiz2.y, 16);
-    fix += lane < 16 ? fix2.x : fix2.y;
-    fiy += lane < 16 ? fiy2.x : fiy2.y;
-    fiz += lane < 16 ? fiz2.x : fiz2.y;
-    if (iValid && (fix != 0.f || fiy != 0.f || fiz != 0.f)) {
+    // the groups hold the same i atoms: after the sum lane l has atom l
+    const float fix = sum_groups(fx, lane), fiy = sum_groups(fy, lane), fiz = sum_groups(fz, lane);
+    if (fix != 0.f || fiy != 0.f || fiz != 0.f) {
+      const int islot = 32 * iBlock + lane;
       red_add(&d.accF[islot], to_fix(fix));
-      red_add(&d.accF[S + islot], to_fix(fiy));
-      red_add(&d.accF[2 * S + islot], to_fix(fiz));
+      red_add(&d.accF[NS + islot], to_fix(fiy));
+      red_add(&d.accF[2 * NS + islot], to_fix(fiz));
       if (!(isfinite(fix) && isfinite(fiy) && isfinite(fiz))) atomicOr(&d.ctr->status, kStatusNonFinite);
     }
-    if (ALCH && bi && fli != 0.f)
-      atomicAdd(reinterpret_cast<unsigned long long *>(&sAccL[bi & 0xFFFF]),
-                static_cast<unsigned long long>(to_fix(fli)));
     if (ENERGY) {
       long long e = ei;
 #pragma unroll
@@ -979,6 +957,7 @@ __global__ void k_finalize(Dev d, bnb_outputs o, int mode) {
 template <int ELEC, int VDW, int ALCH, bool ENERGY, bool COMBINE>
 void launch_t(const KArgs &a, int maxGrid, size_t shmem, cudaStream_t s) {
   auto k = k_pair<ELEC, VDW, ALCH, ENERGY, COMBINE>;
+  shmem += 8 * sizeof(WarpSmem<COMBINE, ALCH>);
   static int perSM = -1, sms = 0;
   static size_t shmemSeen = ~size_t(0);
   if (shmem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);

@@ -385,9 +385,11 @@ int bnb_bias_f32(int blockCount, const float *lambda, const float *fixedBias,
  * CTAs per SM of the persistent grid (0 = as many as fit) and the tail of the
  * work list (0..8): the last tailItems * tilesPerWork candidate tiles of every
  * i block become items of a quarter of the size, taken after all others, so
- * that the persistent warps finish close together (0 = no tail; default 2).
+ * that the persistent warps finish close together (0 = no tail).  Until the
+ * first call the library chooses the tiles per item of each replica from its
+ * size (2, 4 or 8, no tail), and bnb_get_tuning reports those of the largest.
  * A changed tile count or tail takes effect at the next bnb_rebuild.  The
- * split of each block's tiles depends on that block alone, so a replica gives
+ * split of each block's tiles depends on its replica alone, so a replica gives
  * the same bits alone and in a batch at equal settings.  No reference
  * counterpart.
  */
