@@ -253,7 +253,7 @@ __device__ __forceinline__ float2 sel2(bool x, bool y, float2 a, float2 b) {
 // e6 w (a - w b) with w = Rmin^6 r^-3.  Table mode takes (12 c12, 6 c6), combine
 // mode (e6, R) = (sqrt(12 eps_i) sqrt(12 eps_j), Rmin/2_i + Rmin/2_j).  nqq is
 // the negative charge product and nb = -b, so no sign costs an instruction.
-template <bool ENERGY, bool COMBINE>
+template <bool ENERGY, bool COMBINE, bool MSLD>
 __device__ __forceinline__ float2 pme_vfsw_pair2(const PairConst &pc, float2 r2, float2 rinv,
                                                  float2 r, float2 nqq, float2 lj0, float2 lj1, float2 &E) {
   const float2 targ = fma2(f2(pc.pBeta), r, f2(1.0f));
@@ -300,7 +300,10 @@ __device__ __forceinline__ float2 pme_vfsw_pair2(const PairConst &pc, float2 r2,
     const float2 qe_out = mul2(a, sub2(f2(pc.rci3), rinv3));
     const float2 pe2 = sel2(inA, inB, pe_in, pe_out);
     const float2 nqe2 = sel2(inA, inB, qe_in, qe_out);
-    E = fma2(c12, pe2, fma2(c6, nqe2, mul2(mul2(mul2(nqg, f2(-1.f)), p), rinv)));
+    const float2 lj = fma2(c12, pe2, mul2(c6, nqe2));
+    // the order of pair_terms for MSLD pairs, whose large terms may cancel
+    if (MSLD) E = add2(mul2(mul2(mul2(nqq, f2(-1.f)), mul2(p, g)), rinv), lj);
+    else E = fma2(mul2(mul2(nqg, f2(-1.f)), p), rinv, lj);
   }
   // Coulomb part of (dE/dr) r: -qq g (p / r + 2 beta / sqrt(pi))
   return mul2(fma2(nqg, fma2(p, rinv, f2(pc.twoBetaSqrtPi)), flr), rinv2);
@@ -467,6 +470,7 @@ __device__ __forceinline__ void eval_round(const Dev &d, const PairConst &pc, co
       const float2 rinv = make_float2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
       const float2 rr = mul2(r2, rinv);
       float2 s, re = rr, re2 = r2, reinv = rinv, dredr, dredll;
+      bool softA = false, softB = false;
       if (MSLD) {
         s = make_float2(msld_scale(bi[h].x, bj.x, li[h].x, lamj.x), msld_scale(bi[h].y, bj.y, li[h].y, lamj.y));
         dredr = f2(1.f);
@@ -482,8 +486,10 @@ __device__ __forceinline__ void eval_round(const Dev &d, const PairConst &pc, co
             reinv1 = rcp_approx(re1);
             re21 = re1 * re1;
           };
-          if ((bi[h].x | bj.x) != 0 && rr.x < rs.x) soften(rr.x, rs.x, re.x, re2.x, reinv.x, dredr.x, dredll.x);
-          if ((bi[h].y | bj.y) != 0 && rr.y < rs.y) soften(rr.y, rs.y, re.y, re2.y, reinv.y, dredr.y, dredll.y);
+          softA = (bi[h].x | bj.x) != 0 && rr.x < rs.x;
+          softB = (bi[h].y | bj.y) != 0 && rr.y < rs.y;
+          if (softA) soften(rr.x, rs.x, re.x, re2.x, reinv.x, dredr.x, dredll.x);
+          if (softB) soften(rr.y, rs.y, re.y, re2.y, reinv.y, dredr.y, dredll.y);
         }
       }
       float2 fs, E = f2(0.f);
@@ -498,7 +504,7 @@ __device__ __forceinline__ void eval_round(const Dev &d, const PairConst &pc, co
           lj0 = make_float2(vA.x, vB.x);
           lj1 = make_float2(vA.y, vB.y);
         }
-        fs = pme_vfsw_pair2<needE, COMBINE>(pc, re2, reinv, re, nqq, lj0, lj1, E);
+        fs = pme_vfsw_pair2<needE, COMBINE, MSLD>(pc, re2, reinv, re, nqq, lj0, lj1, E);
       } else {
         fs.x = general_pair<ELEC, VDW, needE, COMBINE>(pc, re2.x, reinv.x, re.x, -nqq.x, sLJ, I.row[h].x, tj.x,
                                                        make_float2(I.e6[h].x, I.R[h].x), make_float2(ej.x, Rj.x), E.x);
@@ -509,7 +515,8 @@ __device__ __forceinline__ void eval_round(const Dev &d, const PairConst &pc, co
         // fs = (dE/dr_eff) / r_eff; U = s E(r_eff(r, s)): dU/dr / r = s fs (r_eff / r) dr_eff/dr
         const float2 de = mul2(mul2(fs, re), s);  // s dE/dr_eff
         float2 dl = KIND == 3 ? fma2(de, dredll, E) : E;  // dU/ds
-        fs = KIND == 3 ? mul2(mul2(de, dredr), rinv) : mul2(fs, s);
+        fs = mul2(fs, s);
+        if (KIND == 3) fs = sel2(softA, softB, mul2(mul2(de, dredr), rinv), fs);
         E = mul2(E, s);
         dl = sel2(actA, actB, dl, f2(0.f));
         // dU/dlambda routing, nbdirect.cu:400-415 (block 0 is no variable)
