@@ -80,7 +80,12 @@ struct bnb_handle {
   int pmeOrder = 0, pmeTotalGrid = 0, pmeTotalCplx = 0, pmeMaxCplx = 0;
   std::vector<bnb::PmeRep> pmeRep;
   struct PmePlan { cufftHandle r2c, c2r; int first, count; };
-  std::vector<PmePlan> pmePlans;
+  std::vector<PmePlan> pmePlans;  // cuFFT, where the grids are outside the own transforms' range
+  bool pmeOwn = false;
+  bnb::PmeFftLaunch pmeFft{};
+  int pmeBufElems = 0;
+  float2 *pmeTwiddle_d = nullptr;
+  int2 *pmePlaneMap_d = nullptr, *pmeColMap_d = nullptr;
   bnb::PmeRep *pmeRep_d = nullptr;
   float *pmeMod_d = nullptr, *pmeGrid_d = nullptr;
   float2 *pmeCplx_d = nullptr;
@@ -1295,6 +1300,10 @@ bnb::PmeArgs pme_args(bnb_handle *h, const float *position, const float *lambda)
   a.accE = h->pmeAccE;
   a.done = h->pmeDone;
   a.tric = h->triclinic;
+  a.twiddle = h->pmeTwiddle_d;
+  a.planeMap = h->pmePlaneMap_d;
+  a.colMap = h->pmeColMap_d;
+  a.bufElems = h->pmeBufElems;
   return a;
 }
 }  // namespace
@@ -1335,7 +1344,54 @@ extern "C" int bnb_set_pme(bnb_handle *h, int order, float gridSpace, const int 
     if (gOff > (1LL << 30) || cOff > (1LL << 30)) return BNB_ERR_TOO_LARGE;
   }
   free_pme(h);
+  // Own transforms for all replicas or cuFFT for all.  A plane (one x) of a grid
+  // is transformed by one CTA in shared memory, which ends at about 165^2
+  // points, and the radices are 2 to 8.  Against cuFFT (one evaluation, order
+  // 6): see pmefft.cu.
+  bool own = true;
+  bnb::PmeFftLaunch fl{};
+  std::vector<float2> twiddle;
+  std::vector<int2> planeMap, colMap;
+  int bufElems = 0, maxPlane = 0;
+  for (int r = 0; r < R && own; r++) {
+    const int *K = pr[r].K;
+    int be = 0;
+    for (int k = 0; k < 3; k++) own = own && (pr[r].plan[k] = bnb::pme_fft_plan(K[k])) != 0;
+    const size_t ps = bnb::pme_fft_plane_smem(K, &be), xs = bnb::pme_fft_x_smem(K[0]);
+    own = own && ps <= bnb::kPmeFftSmem && xs <= bnb::kPmeFftSmem;
+    fl.xSmem = std::max(fl.xSmem, xs);
+    bufElems = std::max(bufElems, be);
+    maxPlane = std::max(maxPlane, K[1] * K[2]);
+  }
+  if (own) {
+    size_t tables = 0;
+    for (int r = 0; r < R; r++) {
+      const int *K = pr[r].K;
+      for (int k = 0; k < 3; k++) {
+        pr[r].twOff[k] = (int)twiddle.size();
+        for (int i = 0; i < K[k]; i++) {
+          const double ph = -2.0 * M_PI * i / K[k];
+          twiddle.push_back(make_float2((float)std::cos(ph), (float)std::sin(ph)));
+        }
+      }
+      tables = std::max(tables, (size_t)K[1] + K[2]);
+      for (int x = 0; x < K[0]; x++) planeMap.push_back(make_int2(r, x));
+      for (int c = 0; c < K[1] * (K[2] / 2 + 1); c += bnb::kPmeCols) colMap.push_back(make_int2(r, c));
+    }
+    fl.planes = (int)planeMap.size();
+    fl.colTiles = (int)colMap.size();
+    fl.planeSmem = sizeof(float2) * (2 * (size_t)bufElems + tables);
+    fl.planeThreads = 128;  // about 4 points a thread: the passes are latency in a row
+    while (fl.planeThreads < 1024 && 4 * fl.planeThreads < maxPlane) fl.planeThreads *= 2;
+    own = fl.planeSmem <= bnb::kPmeFftSmem && bnb::pme_fft_setup() == BNB_OK;
+  }
+  if (!own) {
+    twiddle.clear();
+    planeMap.clear();
+    colMap.clear();
+  }
   Arena a;
+  size_t oTw = a.take<float2>(twiddle.size()), oPm = a.take<int2>(planeMap.size()), oCm = a.take<int2>(colMap.size());
   size_t oRep = a.take<bnb::PmeRep>(std::max(R, 1)), oMod = a.take<float>(mOff), oFix = a.take<long long>(gOff),
          oGrid = a.take<float>(gOff), oCplx = a.take<float2>(cOff), oL = a.take<long long>(std::max(h->lamTotal, 1)),
          oE = a.take<long long>(std::max(R, 1)), oDone = a.take<unsigned int>(1);
@@ -1351,6 +1407,9 @@ extern "C" int bnb_set_pme(bnb_handle *h, int order, float gridSpace, const int 
   h->pmeAccL = (long long *)(b + oL);
   h->pmeAccE = (long long *)(b + oE);
   h->pmeDone = (unsigned int *)(b + oDone);
+  h->pmeTwiddle_d = (float2 *)(b + oTw);
+  h->pmePlaneMap_d = (int2 *)(b + oPm);
+  h->pmeColMap_d = (int2 *)(b + oCm);
   std::vector<float> mod(mOff);
   for (int r = 0; r < R; r++) {
     float *m = mod.data() + pr[r].modOff;
@@ -1358,14 +1417,19 @@ extern "C" int bnb_set_pme(bnb_handle *h, int order, float gridSpace, const int 
     pme_moduli(pr[r].K[1], order, pr[r].K[1], m + pr[r].K[0]);
     pme_moduli(pr[r].K[2], order, pr[r].K[2] / 2 + 1, m + pr[r].K[0] + pr[r].K[1]);
   }
-  if (!ok(cudaMemset(base, 0, a.off)) ||
+  auto up = [](void *dst, const void *src, size_t n) {
+    return n == 0 || ok(cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice));
+  };
+  if (!ok(cudaMemset(base, 0, a.off)) || !up(h->pmeTwiddle_d, twiddle.data(), sizeof(float2) * twiddle.size()) ||
+      !up(h->pmePlaneMap_d, planeMap.data(), sizeof(int2) * planeMap.size()) ||
+      !up(h->pmeColMap_d, colMap.data(), sizeof(int2) * colMap.size()) ||
       !ok(cudaMemcpy(h->pmeRep_d, pr.data(), sizeof(bnb::PmeRep) * R, cudaMemcpyHostToDevice)) ||
       !ok(cudaMemcpy(h->pmeMod_d, mod.data(), sizeof(float) * mOff, cudaMemcpyHostToDevice))) {
     free_pme(h);
     return BNB_ERR_CUDA;
   }
-  // one batched plan pair per set of equal grids (contiguous in the layout)
-  for (int i = 0; i < R;) {
+  // cuFFT: one batched plan pair per set of equal grids (contiguous in the layout)
+  for (int i = 0; i < R && !own;) {
     const int r = layout[i];
     int e = i + 1;
     while (e < R && key(layout[e]) == key(r)) e++;
@@ -1388,6 +1452,9 @@ extern "C" int bnb_set_pme(bnb_handle *h, int order, float gridSpace, const int 
     h->pmePlans.push_back(p);
     i = e;
   }
+  h->pmeOwn = own;
+  h->pmeFft = fl;
+  h->pmeBufElems = bufElems;
   h->pmeRep = pr;
   h->pmeOrder = order;
   h->pmeTotalGrid = (int)gOff;
@@ -1417,6 +1484,12 @@ extern "C" int bnb_compute_pme(bnb_handle *h, const float *position, const float
   bnb::PmeArgs a = pme_args(h, position, lambda);
   a.mode = out_mode(calcEnergy);
   if ((rc = bnb::pme_spread(a, s))) return rc;
+  if (h->pmeOwn) {
+    if ((rc = bnb::pme_fft(a, h->pmeFft, s))) return rc;
+    h->launches += 5;
+    return bnb::pme_gather(a, *out, (calcEnergy & 1) != 0, s);
+  }
+  if ((rc = bnb::pme_to_grid(a, s))) return rc;
   for (auto &p : h->pmePlans) {
     const bnb::PmeRep &f = h->pmeRep[p.first];
     if (cufftSetStream(p.r2c, s) != CUFFT_SUCCESS ||

@@ -24,8 +24,10 @@
 // are H^-T m (nbrecip.cu:236-242) and dU/dx = H^-T dU/ds (nbrecip.cu:456-462),
 // with H^-1 as the reference's State::kTricBox_f (state.cxx:485-491).
 // Orthorhombic handles keep the plain per-dimension path.
-// The 3-D FFTs are cuFFT plans (one batched plan per run of consecutive
-// replicas with equal grids), as in the reference.
+// The 3-D transforms are pmefft.cu's, for all replicas at once.  Grids outside
+// its range (a plane above 220 KB of shared memory, about 165^2, or an edge with
+// a prime factor above 5) are cuFFT plans, one batched plan per set of equal
+// grids, as in the reference.
 #include <cuda_runtime.h>
 
 #include "pme.h"
@@ -112,25 +114,6 @@ __device__ __forceinline__ void grid_coords(const PmeArgs &a, const float *x, co
   grid_index(sz * pr.K[2], pr.K[2], i0[2], f[2]);
 }
 
-// H^-1 of a triclinic cell as (xx, xy, xz, yy, yz, zz), FP32 like the
-// reference's kTricBox_f.
-struct RecipCell {
-  float xx, xy, xz, yy, yz, zz;
-};
-__device__ __forceinline__ RecipCell recip_cell(const RepInfo &ri) {
-  const float ax = ri.box[0], by = ri.box[1], cz = ri.box[2];
-  const float bx = ri.tric[0], cx = ri.tric[1], cy = ri.tric[2];
-  const float vinv = 1.f / (ax * by * cz);
-  RecipCell k;
-  k.xx = by * cz * vinv;
-  k.xy = -bx * cz * vinv;
-  k.xz = (bx * cy - by * cx) * vinv;
-  k.yy = cz * ax * vinv;
-  k.yz = -cy * ax * vinv;
-  k.zz = ax * by * vinv;
-  return k;
-}
-
 __device__ __forceinline__ float atom_scale(const PmeArgs &a, int atom, int &block) {
   block = a.siteBlock[atom] & 0xFFFF;
   return (block && a.lambda) ? a.lambda[block] : 1.f;
@@ -193,40 +176,23 @@ __global__ void k_fix_to_grid(PmeArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Convolution: blockIdx.y = replica, threads stride over its half spectrum.
-// FP32 like the reference's kernel (nbrecip.cu:215-256).
+// Convolution between cuFFT transforms: blockIdx.y = replica, threads stride
+// over its half spectrum.
 // ---------------------------------------------------------------------------
 __global__ void k_convolve(PmeArgs a) {
   pdl_wait();
   const int r = blockIdx.y;
   const PmeRep pr = a.prep[r];
   const RepInfo &ri = a.rep[r];
-  const int K0 = pr.K[0], K1 = pr.K[1], K2h = pr.K[2] / 2 + 1;
-  const int n = K0 * K1 * K2h;
-  const float ix = 1.f / ri.box[0], iy = 1.f / ri.box[1], iz = 1.f / ri.box[2];
-  const RecipCell rc = a.tric ? recip_cell(ri) : RecipCell{};
-  const float c = (float)(1.0 / (2.0 * kPi * (double)ri.box[0] * (double)ri.box[1] * (double)ri.box[2]));
-  const float g = (float)(kPi * kPi / ((double)a.beta * (double)a.beta));
-  const float *m0 = a.mod + pr.modOff, *m1 = m0 + K0, *m2 = m1 + K1;
+  const int K1 = pr.K[1], K2h = pr.K[2] / 2 + 1, n = pr.K[0] * K1 * K2h;
+  const InfluenceFn fn(a, pr, ri);
   float2 *spec = a.cplx + pr.cplxOff;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const int k = e % K2h;
     const int row = e / K2h;
     const int j = row % K1;
     const int i = row / K1;
-    const float mi = (float)(2 * i <= K0 ? i : i - K0), mj = (float)(2 * j <= K1 ? j : j - K1), mk = (float)k;
-    float kx, ky, kz;
-    if (!a.tric) {
-      kx = mi * ix;
-      ky = mj * iy;
-      kz = mk * iz;
-    } else {  // k = H^-T m
-      kx = mi * rc.xx;
-      ky = fmaf(mi, rc.xy, mj * rc.yy);
-      kz = fmaf(mi, rc.xz, fmaf(mj, rc.yz, mk * rc.zz));
-    }
-    const float k2 = fmaf(kx, kx, fmaf(ky, ky, kz * kz));
-    const float factor = e == 0 ? 0.f : m0[i] * m1[j] * m2[k] * c * expf(-g * k2) / k2;
+    const float factor = fn(i, j, k);
     float2 v = spec[e];
     v.x *= factor;
     v.y *= factor;
@@ -440,6 +406,10 @@ int pme_spread(const PmeArgs &a, cudaStream_t s) {
       default: return BNB_ERR_ARG;
     }
   }
+  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
+}
+
+int pme_to_grid(const PmeArgs &a, cudaStream_t s) {
   launch_pdl(k_fix_to_grid, grid_of(a.totalGrid, 256), 256, 0, s, a);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
