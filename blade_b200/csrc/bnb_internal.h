@@ -69,6 +69,7 @@ struct RepInfo {          // per replica, device copy in Dev::rep
   int tilesPerWork;       // candidate tiles per work item (1..32)
   int tailTiles;          // last candidate tiles of each i block that go to the tail levels
   float4 shift[14];       // image shift vectors by shift code (kNumShifts)
+  double inv[3];          // 1 / box
 };
 
 // Lattice translation sx A + sy B + sz C in FP32, one rounding per operation

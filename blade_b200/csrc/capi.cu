@@ -323,7 +323,7 @@ bool store_boxes(bnb_handle *h, const float *boxes) {
     for (int k = 0; k < 3; k++)
       if (ri.box[k] != b[k] || ri.tric[k] != t[k]) c = true;
     if (c) {
-      for (int k = 0; k < 3; k++) { ri.box[k] = b[k]; ri.tric[k] = t[k]; }
+      for (int k = 0; k < 3; k++) { ri.box[k] = b[k]; ri.tric[k] = t[k]; ri.inv[k] = 1.0 / (double)b[k]; }
       set_shifts(ri);
       changed = true;
     }
@@ -1299,6 +1299,8 @@ bnb::PmeArgs pme_args(bnb_handle *h, const float *position, const float *lambda)
   a.accL = h->pmeAccL;
   a.accE = h->pmeAccE;
   a.done = h->pmeDone;
+  a.alch = h->alch;
+  a.pi2Beta2 = (float)(M_PI * M_PI / ((double)h->p.betaEwald * (double)h->p.betaEwald));
   a.tric = h->triclinic;
   a.twiddle = h->pmeTwiddle_d;
   a.planeMap = h->pmePlaneMap_d;
@@ -1346,8 +1348,8 @@ extern "C" int bnb_set_pme(bnb_handle *h, int order, float gridSpace, const int 
   free_pme(h);
   // Own transforms for all replicas or cuFFT for all.  A plane (one x) of a grid
   // is transformed by one CTA in shared memory, which ends at about 165^2
-  // points, and the radices are 2 to 8.  Against cuFFT (one evaluation, order
-  // 6): see pmefft.cu.
+  // points, and the radices are 2 to 8.  Faster than cuFFT at every size it
+  // takes (pmefft.cu).
   bool own = true;
   bnb::PmeFftLaunch fl{};
   std::vector<float2> twiddle;
@@ -1381,8 +1383,13 @@ extern "C" int bnb_set_pme(bnb_handle *h, int order, float gridSpace, const int 
     fl.planes = (int)planeMap.size();
     fl.colTiles = (int)colMap.size();
     fl.planeSmem = sizeof(float2) * (2 * (size_t)bufElems + tables);
-    fl.planeThreads = 128;  // about 4 points a thread: the passes are latency in a row
-    while (fl.planeThreads < 1024 && 4 * fl.planeThreads < maxPlane) fl.planeThreads *= 2;
+    // one CTA per SM at most: about 4 points a thread, the passes are latency in
+    // a row (64^3: 52 -> 47 us an evaluation against 16 points); more planes
+    // than SMs: 16, so that CTAs share an SM (8 replicas of 36^3 to 54^3: a step
+    // 370 -> 359 us against 4)
+    const int points = fl.planes <= 148 ? 4 : 16;
+    fl.planeThreads = 128;
+    while (fl.planeThreads < 1024 && points * fl.planeThreads < maxPlane) fl.planeThreads *= 2;
     own = fl.planeSmem <= bnb::kPmeFftSmem && bnb::pme_fft_setup() == BNB_OK;
   }
   if (!own) {

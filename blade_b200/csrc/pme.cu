@@ -13,10 +13,11 @@
 // Differences by design:
 //   * the charge grid accumulates in int64 fixed point (2^-32), so the grid,
 //     and with it every output, is identical run to run;
-//   * u is formed in FP64 and wrapped with floor/mod, so any unwrapped
-//     coordinate lands on the right grid point;
-//   * lanes of an atom's 8-lane group own z offsets (contiguous grid
-//     addresses within one instruction) instead of x/y/z parity classes;
+//   * u is formed in FP64 and wrapped, so any unwrapped coordinate lands on
+//     the right grid point;
+//   * lanes own z offsets (contiguous grid addresses within one instruction)
+//     instead of x/y/z parity classes, and the atoms of a molecule are spread
+//     together;
 //   * R replicas with their own grids in one launch per phase.
 // Triclinic cells (the reference's flagBox branch): the fractional
 // coordinates s = H^-1 x of the cell matrix H (columns A, B, C) replace x / L
@@ -77,41 +78,23 @@ __device__ __forceinline__ void bspline(float f, float (&w)[ORDER], float (&dw)[
   }
 }
 
-// Grid coordinate of one dimension: first grid index (mod K) and fraction.
-__device__ __forceinline__ void grid_coord(float x, int K, float L, int &i0, float &frac) {
-  const double u = (double)x * (double)K / (double)L;
-  const double u0 = floor(u);
-  frac = (float)(u - u0);
-  double m = u0 - (double)K * floor(u0 / (double)K);
-  i0 = (int)m;
-  if (i0 >= K) i0 -= K;  // m rounds to K only when u0 is a tiny negative multiple
-  if (i0 < 0) i0 += K;
-}
-
-// Grid index (mod K) and fraction of a coordinate already in grid units.
-__device__ __forceinline__ void grid_index(double u, int K, int &i0, float &frac) {
-  const double u0 = floor(u);
-  frac = (float)(u - u0);
-  double m = u0 - (double)K * floor(u0 / (double)K);
-  i0 = (int)m;
-  if (i0 >= K) i0 -= K;
-  if (i0 < 0) i0 += K;
-}
-
-// Grid coordinates of an atom in its replica's cell (both box types).
-__device__ __forceinline__ void grid_coords(const PmeArgs &a, const float *x, const PmeRep &pr, const RepInfo &ri,
-                                            int (&i0)[3], float (&f)[3]) {
+// First grid index (mod K) and fraction of an atom along dimension `dim` of its
+// replica's cell.  The fractional coordinate is formed in FP64 and reduced to
+// [0, 1) before it is scaled, so any unwrapped coordinate lands on its grid point.
+__device__ __forceinline__ void grid_coord(const PmeArgs &a, const float *x, int K, const RepInfo &ri, int dim,
+                                           int &i0, float &frac) {
+  double f;
   if (!a.tric) {
-    for (int d = 0; d < 3; d++) grid_coord(x[d], pr.K[d], ri.box[d], i0[d], f[d]);
-    return;
+    f = (double)x[dim] * ri.inv[dim];
+  } else {  // box = (A_x, B_y, C_z), tric = (B_x, C_x, C_y)
+    const double sz = (double)x[2] * ri.inv[2];
+    const double sy = ((double)x[1] - (double)ri.tric[2] * sz) * ri.inv[1];
+    f = dim == 2 ? sz : (dim == 1 ? sy : ((double)x[0] - (double)ri.tric[0] * sy - (double)ri.tric[1] * sz) * ri.inv[0]);
   }
-  // box = (A_x, B_y, C_z), tric = (B_x, C_x, C_y)
-  const double sz = (double)x[2] / (double)ri.box[2];
-  const double sy = ((double)x[1] - (double)ri.tric[2] * sz) / (double)ri.box[1];
-  const double sx = ((double)x[0] - (double)ri.tric[0] * sy - (double)ri.tric[1] * sz) / (double)ri.box[0];
-  grid_index(sx * pr.K[0], pr.K[0], i0[0], f[0]);
-  grid_index(sy * pr.K[1], pr.K[1], i0[1], f[1]);
-  grid_index(sz * pr.K[2], pr.K[2], i0[2], f[2]);
+  const double u = (f - floor(f)) * (double)K, u0 = floor(u);
+  frac = (float)(u - u0);
+  i0 = (int)u0;
+  if ((unsigned)i0 >= (unsigned)K) i0 = 0;  // f rounds to 1 (a tiny negative number), or is no number
 }
 
 __device__ __forceinline__ float atom_scale(const PmeArgs &a, int atom, int &block) {
@@ -120,47 +103,142 @@ __device__ __forceinline__ float atom_scale(const PmeArgs &a, int atom, int &blo
 }
 
 // ---------------------------------------------------------------------------
-// Spread: 8 lanes per atom; lane g < ORDER owns z offset g and visits the
-// ORDER x ORDER (x, y) offsets.
+// Spread.  A warp takes 9 consecutive atoms: lanes 3 j + dim evaluate their
+// splines (one coordinate and one spline per warp instead of three per atom)
+// into shared memory; then runs of up to 4 neighbouring atoms whose first grid
+// points lie within (8 - ORDER) / 2 of the run's first atom's (the atoms of a
+// molecule) are spread together over a box of 8 points an edge, lane = 4 rows of
+// y x 8 z, two rows of y per lane: the atoms' fixed-point values of a point are
+// summed in registers and added to the grid once.  The values and the sums are
+// those of one addition per atom.
+//
+// Bound by the L2's atomic additions (0.52 T/s of 64 bits) and the issue of the
+// fixed-point conversions: one addition per atom and point is 216 an atom at
+// order 6; a water's three atoms together touch about 330 points, not 648.
+// Measured at order 6: 192,000 atoms 80 -> 50 us, 20,577 atoms 16 -> 13.6 us.
 // ---------------------------------------------------------------------------
+constexpr int kSpreadAtoms = 9;
+
+// The box of one run of NA atoms, x plane by x plane.  bx, by, bz: weights of the
+// box's points by atom (.x .. .w), zero outside an atom's own points; bz carries
+// the charge in fixed-point units.
+template <int NA>
+__device__ __forceinline__ void spread_box(const float4 *bx, float4 by0, float4 by1, float4 bz, long long *base,
+                                           int row0, int row1, int x0, int K0, int plane) {
+  auto get = [](const float4 &v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); };
+#pragma unroll 2
+  for (int x = 0; x < 8; x++) {
+    const float4 w = bx[x];
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < NA; k++) any = any || get(w, k) != 0.f;
+    if (!any) continue;  // uniform
+    long long s0 = 0, s1 = 0;
+#pragma unroll
+    for (int k = 0; k < NA; k++) {
+      const float q = get(bz, k) * get(w, k);
+      s0 += __float2ll_rn(q * get(by0, k));
+      s1 += __float2ll_rn(q * get(by1, k));
+    }
+    int ix = x0 + x;
+    if (ix >= K0) ix -= K0;
+    if (ix >= K0) ix -= K0;  // a box may be longer than a short edge
+    long long *p = base + (size_t)ix * plane;
+    if (s0) red_add(p + row0, s0);
+    if (s1) red_add(p + row1, s1);
+  }
+}
+
 template <int ORDER>
 __global__ void __launch_bounds__(256) k_spread(PmeArgs a) {
   pdl_wait();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int atom = t >> 3, g = t & 7;
-  if (atom >= a.N || g >= ORDER) return;
-  const int r = a.atomRep[atom];
-  const PmeRep pr = a.prep[r];
-  const RepInfo &ri = a.rep[r];
-  int block;
-  const float qe = a.q[atom] * atom_scale(a, atom, block);
-  if (qe == 0.f) return;
-  float wx[ORDER], wy[ORDER], wz[ORDER], d[ORDER];
-  int i0[3];
-  float f[3];
-  grid_coords(a, a.x + 3 * atom, pr, ri, i0, f);
-  const int ix0 = i0[0], iy0 = i0[1], iz0 = i0[2];
-  bspline<ORDER>(f[0], wx, d);
-  bspline<ORDER>(f[1], wy, d);
-  bspline<ORDER>(f[2], wz, d);
-  float wzg = wz[0];
+  constexpr int RANGE = (8 - ORDER) / 2;
+  __shared__ float sW[8][kSpreadAtoms][3][8];
+  __shared__ float4 sB[8][3][8];  // a run's box: [dim][point], component = atom
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int first = (blockIdx.x * 8 + wp) * kSpreadAtoms;
+  if (first >= a.N) return;  // uniform per warp
+  const int cnt = a.N - first < kSpreadAtoms ? a.N - first : kSpreadAtoms;
+  int mine = 0;  // lane 3 j + dim: first grid index of atom j along dim
+  {
+    const int j = lane / 3, dim = lane - 3 * j;
+    if (lane < 3 * cnt) {
+      const int atom = first + j, r = a.atomRep[atom];
+      float frac, w[ORDER], d[ORDER];
+      grid_coord(a, a.x + 3 * atom, a.prep[r].K[dim], a.rep[r], dim, mine, frac);
+      bspline<ORDER>(frac, w, d);
 #pragma unroll
-  for (int k = 1; k < ORDER; k++) wzg = g == k ? wz[k] : wzg;
-  const float qz = qe * wzg;
-  int iz = iz0 + g;
-  if (iz >= pr.K[2]) iz -= pr.K[2];
-  long long *base = a.qfix + pr.gridOff;
-#pragma unroll
-  for (int tx = 0; tx < ORDER; tx++) {
-    int ix = ix0 + tx;
-    if (ix >= pr.K[0]) ix -= pr.K[0];
-    const float qx = qz * wx[tx];
-#pragma unroll
-    for (int ty = 0; ty < ORDER; ty++) {
-      int iy = iy0 + ty;
-      if (iy >= pr.K[1]) iy -= pr.K[1];
-      red_add(base + ((size_t)ix * pr.K[1] + iy) * pr.K[2] + iz, to_fix(qx * wy[ty]));
+      for (int k = 0; k < ORDER; k++) sW[wp][j][dim][k] = w[k];
     }
+  }
+  // lane j: atom j's first grid indices, charge and replica
+  int g[3], rep = -1;
+#pragma unroll
+  for (int k = 0; k < 3; k++) g[k] = __shfl_sync(kFull, mine, 3 * lane + k);
+  float q = 0.f;
+  if (lane < cnt) {
+    int block;
+    q = a.q[first + lane] * atom_scale(a, first + lane, block);
+    rep = a.atomRep[first + lane];
+  }
+  __syncwarp();
+  const int z = lane & 7, y = lane >> 3;
+  unsigned left = __ballot_sync(kFull, q != 0.f);
+  while (left) {
+    const int h = __ffs(left) - 1;
+    const int r = __shfl_sync(kFull, rep, h);
+    const PmeRep &pr = a.prep[r];
+    const int K0 = pr.K[0], K1 = pr.K[1], K2 = pr.K[2];
+    // offsets from the run's first atom; the run ends at the first that is not near
+    int c[3], e[3];
+    bool near = rep == r;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const int K = pr.K[k];
+      c[k] = __shfl_sync(kFull, g[k], h);
+      e[k] = g[k] - c[k];
+      e[k] = 2 * e[k] > K ? e[k] - K : (2 * e[k] < -K ? e[k] + K : e[k]);
+      near = near && e[k] >= -RANGE && e[k] <= RANGE;
+    }
+    const unsigned run = __ballot_sync(kFull, near) >> h;
+    const int len = __ffs(~run) - 1, n = len < 4 ? len : 4;
+    {  // lane 8 k + i: the weights of atom h + k at point i of the box
+      const int k = lane >> 3, i = lane & 7, at = (h + k) & 31;
+      const int e0 = __shfl_sync(kFull, e[0], at), e1 = __shfl_sync(kFull, e[1], at), e2 = __shfl_sync(kFull, e[2], at);
+      const float qk = __shfl_sync(kFull, q, at) * kFixScaleF;  // a power of two: exact
+      float w0 = 0.f, w1 = 0.f, w2 = 0.f;
+      if (k < n) {
+        const float(&w)[3][8] = sW[wp][h + k];
+        const int t0 = i - RANGE - e0, t1 = i - RANGE - e1, t2 = i - RANGE - e2;
+        if ((unsigned)t0 < (unsigned)ORDER) w0 = w[0][t0];
+        if ((unsigned)t1 < (unsigned)ORDER) w1 = w[1][t1];
+        if ((unsigned)t2 < (unsigned)ORDER) w2 = qk * w[2][t2];
+      }
+      __syncwarp();  // the run before has been read
+      reinterpret_cast<float *>(&sB[wp][0][i])[k] = w0;
+      reinterpret_cast<float *>(&sB[wp][1][i])[k] = w1;
+      reinterpret_cast<float *>(&sB[wp][2][i])[k] = w2;
+      __syncwarp();
+    }
+    // grid index of a box point; a box may be longer than a short edge
+    auto wrapped = [](int i, int K) {
+      if (i < 0) i += K;
+      if (i >= K) i -= K;
+      if (i >= K) i -= K;
+      return i;
+    };
+    int x0 = c[0] - RANGE;
+    if (x0 < 0) x0 += K0;
+    long long *base = a.qfix + pr.gridOff + wrapped(c[2] - RANGE + z, K2);
+    const int row0 = wrapped(c[1] - RANGE + y, K1) * K2, row1 = wrapped(c[1] - RANGE + y + 4, K1) * K2;
+    const float4 by0 = sB[wp][1][y], by1 = sB[wp][1][y + 4], bz = sB[wp][2][z];
+    switch (n) {
+      case 1: spread_box<1>(sB[wp][0], by0, by1, bz, base, row0, row1, x0, K0, K1 * K2); break;
+      case 2: spread_box<2>(sB[wp][0], by0, by1, bz, base, row0, row1, x0, K0, K1 * K2); break;
+      case 3: spread_box<3>(sB[wp][0], by0, by1, bz, base, row0, row1, x0, K0, K1 * K2); break;
+      default: spread_box<4>(sB[wp][0], by0, by1, bz, base, row0, row1, x0, K0, K1 * K2); break;
+    }
+    left &= ~(((1u << n) - 1u) << h);
   }
 }
 
@@ -236,116 +314,136 @@ __device__ void finalize_if_last(const PmeArgs &a, const bnb_outputs &o, bool en
 }
 
 // ---------------------------------------------------------------------------
-// Gather: same lane layout as the spread; the 8 lanes of an atom reduce with
-// xor shuffles, lane 0 of the group writes the atom's outputs.
+// Gather.  A warp takes 8 atoms: lanes 3 j + dim evaluate their splines into
+// shared memory, then 8 lanes per atom gather, 4 atoms at a time: lane g owns z
+// offset g and visits the ORDER x ORDER (x, y) offsets; the 8 lanes of an atom
+// reduce with xor shuffles and lanes 0-2 write its force.
+//
+// Bound by the latency of its loads, so by the warps in flight: 64 registers (4
+// CTAs per SM) 138 us an evaluation of 192,000 atoms, 80 registers 151, 48 with
+// spills 162.  Gathering a molecule's atoms together, as the spread does, loads
+// half as much and was slower (150 us): it is not the loads' number that bounds.
 // ---------------------------------------------------------------------------
+constexpr int kGatherAtoms = 8;
 template <int ORDER, bool ENERGY>
-__global__ void __launch_bounds__(256) k_gather(PmeArgs a, bnb_outputs o) {
+__global__ void __launch_bounds__(256, 4) k_gather(PmeArgs a, bnb_outputs o) {
   pdl_wait();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  const int atom = t >> 3, g = t & 7;
-  const bool valid = atom < a.N;
-  float phi = 0.f, gx = 0.f, gy = 0.f, gz = 0.f, qe = 0.f, qraw = 0.f;
-  int r = 0, block = 0;
-  PmeRep pr{};
-  if (valid) {
-    r = a.atomRep[atom];
-    pr = a.prep[r];
-    const RepInfo &ri = a.rep[r];
-    qraw = a.q[atom];
-    qe = qraw * atom_scale(a, atom, block);
-    if (g < ORDER) {
-      float wx[ORDER], wy[ORDER], wz[ORDER], dx[ORDER], dy[ORDER], dz[ORDER];
-      int i0[3];
-      float f[3];
-      grid_coords(a, a.x + 3 * atom, pr, ri, i0, f);
-      const int ix0 = i0[0], iy0 = i0[1], iz0 = i0[2];
-      bspline<ORDER>(f[0], wx, dx);
-      bspline<ORDER>(f[1], wy, dy);
-      bspline<ORDER>(f[2], wz, dz);
-      float wzg = wz[0], dzg = dz[0];
+  __shared__ float sW[8][kGatherAtoms][3][8], sD[8][kGatherAtoms][3][8];
+  __shared__ int sI[8][kGatherAtoms][4];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, g = lane & 7;
+  const int first = (blockIdx.x * 8 + wp) * kGatherAtoms;
+  {
+    const int j = lane / 3, dim = lane - 3 * j, atom = first + j;
+    if (lane < 3 * kGatherAtoms && atom < a.N) {
+      const int r = a.atomRep[atom];
+      int i0;
+      float frac, w[ORDER], d[ORDER];
+      grid_coord(a, a.x + 3 * atom, a.prep[r].K[dim], a.rep[r], dim, i0, frac);
+      bspline<ORDER>(frac, w, d);
 #pragma unroll
-      for (int k = 1; k < ORDER; k++) {
-        wzg = g == k ? wz[k] : wzg;
-        dzg = g == k ? dz[k] : dzg;
+      for (int k = 0; k < ORDER; k++) {
+        sW[wp][j][dim][k] = w[k];
+        sD[wp][j][dim][k] = d[k];
       }
-      int iz = iz0 + g;
-      if (iz >= pr.K[2]) iz -= pr.K[2];
-      const float *base = a.grid + pr.gridOff;
+      sI[wp][j][dim] = i0;
+      if (dim == 0) sI[wp][j][3] = r;
+    }
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int half = 0; half < 2; half++) {
+    const int j = 4 * half + (lane >> 3), atom = first + j;
+    const bool valid = atom < a.N;
+    float phi = 0.f, gx = 0.f, gy = 0.f, gz = 0.f, qe = 0.f, qraw = 0.f;
+    int r = 0, block = 0;
+    PmeRep pr{};
+    if (valid) {
+      r = sI[wp][j][3];
+      pr = a.prep[r];
+      qraw = a.q[atom];
+      qe = qraw * atom_scale(a, atom, block);
+    }
+    if (valid && g < ORDER) {
+      const int K0 = pr.K[0], K1 = pr.K[1], K2 = pr.K[2];
+      int iz = sI[wp][j][2] + g;
+      if (iz >= K2) iz -= K2;
+      const float *base = a.grid + pr.gridOff + iz;
+      int oy[ORDER];
+      float wy[ORDER], dy[ORDER];
+#pragma unroll
+      for (int ty = 0; ty < ORDER; ty++) {
+        int iy = sI[wp][j][1] + ty;
+        if (iy >= K1) iy -= K1;
+        oy[ty] = iy * K2;
+        wy[ty] = sW[wp][j][1][ty];
+        dy[ty] = sD[wp][j][1][ty];
+      }
 #pragma unroll
       for (int tx = 0; tx < ORDER; tx++) {
-        int ix = ix0 + tx;
-        if (ix >= pr.K[0]) ix -= pr.K[0];
+        int ix = sI[wp][j][0] + tx;
+        if (ix >= K0) ix -= K0;
+        const float *plane = base + (size_t)ix * (K1 * K2);
+        const float wx = sW[wp][j][0][tx], dx = sD[wp][j][0][tx];
         float p = 0.f, py = 0.f;  // sum over y of P wy, P dy
 #pragma unroll
         for (int ty = 0; ty < ORDER; ty++) {
-          int iy = iy0 + ty;
-          if (iy >= pr.K[1]) iy -= pr.K[1];
-          const float P = __ldg(base + ((size_t)ix * pr.K[1] + iy) * pr.K[2] + iz);
+          const float P = __ldg(plane + oy[ty]);
           p = fmaf(P, wy[ty], p);
           py = fmaf(P, dy[ty], py);
         }
-        phi = fmaf(wx[tx], p, phi);
-        gx = fmaf(dx[tx], p, gx);
-        gy = fmaf(wx[tx], py, gy);
+        phi = fmaf(wx, p, phi);
+        gx = fmaf(dx, p, gx);
+        gy = fmaf(wx, py, gy);
       }
-      gz = phi * dzg;
-      phi *= wzg;
-      gx *= wzg;
-      gy *= wzg;
+      const float wz = sW[wp][j][2][g];
+      gz = phi * sD[wp][j][2][g];
+      phi *= wz;
+      gx *= wz;
+      gy *= wz;
     }
-  }
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) {
-    phi += __shfl_xor_sync(kFull, phi, o);
-    gx += __shfl_xor_sync(kFull, gx, o);
-    gy += __shfl_xor_sync(kFull, gy, o);
-    gz += __shfl_xor_sync(kFull, gz, o);
-  }
-  float e = 0.f;
-  if (valid && g == 0) {
-    const RepInfo &ri = a.rep[r];
-    const float c = 2.f * qe;
-    float fx, fy, fz;
-    if (!a.tric) {
-      fx = c * gx * ((float)pr.K[0] / ri.box[0]);
-      fy = c * gy * ((float)pr.K[1] / ri.box[1]);
-      fz = c * gz * ((float)pr.K[2] / ri.box[2]);
-    } else {  // dU/dx = H^-T dU/ds
-      const RecipCell k = recip_cell(ri);
-      const float hx = c * gx * (float)pr.K[0], hy = c * gy * (float)pr.K[1], hz = c * gz * (float)pr.K[2];
-      fx = hx * k.xx;
-      fy = fmaf(hx, k.xy, hy * k.yy);
-      fz = fmaf(hx, k.xz, fmaf(hy, k.yz, hz * k.zz));
+    for (int q = 4; q > 0; q >>= 1) {
+      phi += __shfl_xor_sync(kFull, phi, q);
+      gx += __shfl_xor_sync(kFull, gx, q);
+      gy += __shfl_xor_sync(kFull, gy, q);
+      gz += __shfl_xor_sync(kFull, gz, q);
     }
-    if (o.force64) {
-      out64(&o.force64[3 * atom], fx, a.mode);
-      out64(&o.force64[3 * atom + 1], fy, a.mode);
-      out64(&o.force64[3 * atom + 2], fz, a.mode);
+    if (valid && g < 3) {  // lane g: component g
+      const RepInfo &ri = a.rep[r];
+      const float c = 2.f * qe;
+      float f;
+      if (!a.tric) {
+        f = c * (g == 0 ? gx : (g == 1 ? gy : gz)) * ((float)pr.K[g] / ri.box[g]);
+      } else {  // dU/dx = H^-T dU/ds
+        const RecipCell k = recip_cell(ri);
+        const float hx = c * gx * (float)pr.K[0], hy = c * gy * (float)pr.K[1], hz = c * gz * (float)pr.K[2];
+        f = g == 0 ? hx * k.xx : (g == 1 ? fmaf(hx, k.xy, hy * k.yy) : fmaf(hx, k.xz, fmaf(hy, k.yz, hz * k.zz)));
+      }
+      if (o.force64) out64(&o.force64[3 * atom + g], f, a.mode);
+      if (o.force) out32(&o.force[3 * atom + g], f, a.mode);
     }
-    if (o.force) {
-      out32(&o.force[3 * atom], fx, a.mode);
-      out32(&o.force[3 * atom + 1], fy, a.mode);
-      out32(&o.force[3 * atom + 2], fz, a.mode);
+    float e = 0.f;
+    if (valid && g == 0) {
+      if (block) red_add(&a.accL[block], to_fix(2.f * qraw * phi));
+      if (ENERGY) e = qe * phi;
     }
-    if (block) red_add(&a.accL[block], to_fix(2.f * qraw * phi));
-    if (ENERGY) e = qe * phi;
-  }
-  if (ENERGY) {
-    // one atomic per warp when its 4 atoms share a replica
-    const int r0 = __shfl_sync(kFull, r, 0);
-    const bool same = __all_sync(kFull, !valid || r == r0);
-    long long ef = to_fix(e);
-    if (same) {
+    if (ENERGY) {
+      // one atomic per warp when its 4 atoms share a replica
+      const int r0 = __shfl_sync(kFull, r, 0);
+      const bool same = __all_sync(kFull, !valid || r == r0);
+      long long ef = to_fix(e);
+      if (same) {
 #pragma unroll
-      for (int o2 = 16; o2 > 0; o2 >>= 1) ef += __shfl_xor_sync(kFull, ef, o2);
-      if (lane == 0 && ef) red_add(&a.accE[r0], ef);
-    } else if (ef) {
-      red_add(&a.accE[r], ef);
+        for (int o2 = 16; o2 > 0; o2 >>= 1) ef += __shfl_xor_sync(kFull, ef, o2);
+        if (lane == 0 && ef) red_add(&a.accE[r0], ef);
+      } else if (ef) {
+        red_add(&a.accE[r], ef);
+      }
     }
   }
-  finalize_if_last(a, o, ENERGY);
+  // without energy and MSLD atoms there is nothing to wait for: the sums are zero
+  if (ENERGY || a.alch) finalize_if_last(a, o, ENERGY);
+  else if (blockIdx.x == 0) finalize_outputs(a, o, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -398,7 +496,7 @@ inline int grid_of(long long threads, int block) {
 
 int pme_spread(const PmeArgs &a, cudaStream_t s) {
   if (a.N > 0) {
-    const int grid = (int)((8LL * a.N + 255) / 256);
+    const int grid = (a.N + 8 * kSpreadAtoms - 1) / (8 * kSpreadAtoms);
     switch (a.order) {
       case 4: launch_pdl(k_spread<4>, grid, 256, 0, s, a); break;
       case 6: launch_pdl(k_spread<6>, grid, 256, 0, s, a); break;
@@ -423,7 +521,7 @@ int pme_convolve(const PmeArgs &a, cudaStream_t s) {
 
 int pme_gather(const PmeArgs &a, const bnb_outputs &o, bool energy, cudaStream_t s) {
   if (a.N > 0) {
-    const int grid = (int)((8LL * a.N + 255) / 256);
+    const int grid = (a.N + 8 * kGatherAtoms - 1) / (8 * kGatherAtoms);
     switch (a.order * 2 + (energy ? 1 : 0)) {
       case 8: launch_pdl(k_gather<4, false>, grid, 256, 0, s, a, o); break;
       case 9: launch_pdl(k_gather<4, true>, grid, 256, 0, s, a, o); break;

@@ -16,13 +16,13 @@ struct PmeRep {            // per replica: grid sizes and offsets into the conca
   uint32_t plan[3];        // radices of each dimension, 4 bits each, first pass lowest
 };
 
-constexpr int kPmeCols = 16;                  // columns per CTA of the transform along x
+constexpr int kPmeCols = 8;                   // columns per CTA of the transform along x
 constexpr size_t kPmeFftSmem = 220 * 1024;    // most shared memory of a transform CTA
 
 struct PmeArgs {
   int N, R, lamTotal, order;
   int totalGrid, totalCplx, maxCplx;  // maxCplx: largest half spectrum of one replica
-  float beta;
+  float beta, pi2Beta2;    // pi2Beta2: pi^2 / beta^2
   const float *x;          // [3N] caller positions (State::position_fd)
   const float *lambda;     // [lamTotal] or null (every scale 1)
   const float *q;          // [N] charge * sqrt(kElectric)
@@ -38,6 +38,7 @@ struct PmeArgs {
   long long *accE;         // [R]
   unsigned int *done;      // CTAs finished in the current gather / self launch (zero between launches)
   int mode;                // BNB_OUT_SET / BNB_OUT_ADD64 bits of the call
+  int alch;                // some atom belongs to an MSLD block
   int tric;                // boxes are triclinic cells (RepInfo::box and ::tric)
   // own transforms (pmefft.cu)
   const float2 *twiddle;   // exp(-2 pi i k / K) per replica and dimension
@@ -83,13 +84,13 @@ struct InfluenceFn {
     constexpr double pi = 3.14159265358979323846;
     K0 = pr.K[0];
     K1 = pr.K[1];
-    ix = 1.f / ri.box[0];
-    iy = 1.f / ri.box[1];
-    iz = 1.f / ri.box[2];
+    ix = (float)ri.inv[0];
+    iy = (float)ri.inv[1];
+    iz = (float)ri.inv[2];
     tric = a.tric != 0;
     rc = tric ? recip_cell(ri) : RecipCell{};
-    c = (float)(1.0 / (2.0 * pi * (double)ri.box[0] * (double)ri.box[1] * (double)ri.box[2]));
-    g = (float)(pi * pi / ((double)a.beta * (double)a.beta));
+    c = (float)(ri.inv[0] * ri.inv[1] * ri.inv[2] * (0.5 / pi));
+    g = a.pi2Beta2;
     m0 = a.mod + pr.modOff;
     m1 = m0 + K0;
     m2 = m1 + K1;
