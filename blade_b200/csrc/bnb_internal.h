@@ -17,7 +17,6 @@
 namespace bnb {
 
 constexpr int kNumShifts = 14;        // own image + 13 half-shell images
-constexpr int kExclBlk = 16;          // exclusion-partner blocks listed per block
 constexpr int kTilesPerWork = 8;      // most candidate tiles per pair-kernel work item by default
 constexpr int kMinAutoTiles = 2;      // fewest by default (replica_tiles)
 constexpr int kMinTilesPerWork = 1;   // smallest setting (sizes the work-item capacity)
@@ -97,16 +96,14 @@ __host__ __device__ __forceinline__ float3 lattice_shift(const float *box, const
 // Device-side scalar counters written by the list builder.
 struct Counters {
   int blockCount;
-  int candCount;
-  int maskCount;
-  int workCount;
+  int candCount;           // candidates, masks and work items the list needs (above the
+  int maskCount;           // capacity when the status word reports the overflow)
+  int work[2];             // full-size items, tail items
   int status;
   int workNext;            // dynamic work-item counter of the pair kernel
   int orderValid;          // Dev::order holds the measured longest-first order of the work items
-  int pad;
+  int wide, wideBin;       // an atom lies outside its column (list, binning under way)
   unsigned long long pairCount;
-  int levelCount[kWorkLevels];  // work items per level of the work list (rebuild)
-  int levelFill[kWorkLevels];   // items written per level (rebuild)
 };
 
 struct Dev {
@@ -127,10 +124,10 @@ struct Dev {
   int *wrap;               // [N] packed integer image shift
   int *atomCol;            // [N]
   uint32_t *atomZKey;      // [N]
+  int *atomRank;           // [N] place of the atom in its column's bucket
   int *colCount;           // [totalCols]
   int *colStartAtom;       // [totalCols+1]
   int *colStartBlock;      // [totalCols+1]
-  int *colFill;            // [totalCols]
   int *bucket;             // [N]
   int *sortedAtom;         // [N]
   int *blockBounds;        // [maxBlocks+1]
@@ -143,19 +140,13 @@ struct Dev {
   float2 *slotLj;          // [32*maxBlocks] combine mode: ljType of the slot's type
   int *slotSiteBlock;      // [32*maxBlocks]
   uint32_t *colKey;        // [6*totalCols] column AABB (union of its blocks) as order-preserving keys
-  int *exclBlk;            // [maxBlocks*kExclBlk] distinct blocks holding excluded partners
-  int *exclBlkCount;       // [maxBlocks] entries in exclBlk, -1 = more than kExclBlk
-  int *cullCount;          // [maxBlocks*kNumShifts]
-  int *cullOffset;         // [maxBlocks*kNumShifts+1]
   int4 *cand;              // [capCand] (jBlock, shiftCode, maskIdx, iBlock)
-  int *candFlag;           // [capCand]
-  int *candMaskOff;        // [capCand+1]
   uint32_t *masks;         // [capMask*32] word of j atom l: bit i clear = excluded from i atom i
-  int *candStart;          // [maxBlocks+1]
-  int2 *work;              // [capWork] (iBlock | tiles << 22, candidate start)
-  unsigned int *itemCost;  // [capWork] clock cycles of each work item in the last pair launch
-  int *order;              // [capWork] work items by decreasing measured cost
-  int *scanPartial;        // scratch for multi-CTA scans
+  int *candStart;          // [maxBlocks] first candidate of the block (blocks in any order)
+  int *candNum;            // [maxBlocks] its candidates
+  int2 *work;              // [2*capWork] (iBlock | tiles << 22, candidate start); tail items from capWork on
+  unsigned int *itemCost;  // [2*capWork] by place in the sequence full-size items, tail items: clock cycles of each work item in the last pair launch
+  int *order;              // [2*capWork] work items by decreasing measured cost
   // --- per-step buffers -----------------------------------------------------
   float4 *xyzq;            // [32*maxBlocks]
   float4 *bmin, *bmax;     // [maxBlocks]

@@ -95,7 +95,7 @@ struct bnb_handle {
 
 namespace {
 
-// Largest list capacity: the three-pass scan handles up to 4096 x 4096 items.
+// Largest list capacity.
 constexpr long long kCapLimit = 4096LL * 4096LL;
 constexpr int kProfSlots = 4096;
 
@@ -198,21 +198,18 @@ int alloc_list(bnb_handle *h) {
   Arena a;
   size_t o_wrap = a.take<int>(N), o_col = a.take<int>(N), o_z = a.take<uint32_t>(N);
   size_t o_cc = a.take<int>(C), o_csa = a.take<int>(C + 1), o_csb = a.take<int>(C + 1),
-         o_cf = a.take<int>(C), o_colrep = a.take<int>(C);
+         o_rank = a.take<int>(N), o_colrep = a.take<int>(C);
   size_t o_bucket = a.take<int>(N), o_sorted = a.take<int>(N);
   size_t o_bb = a.take<int>(MB + 1), o_brep = a.take<int>(MB), o_rbs = a.take<int>(h->R + 1);
   size_t o_slotA = a.take<int>(32 * MB), o_atomSlot = a.take<int>(N), o_slotQ = a.take<float>(32 * MB),
          o_slotT = a.take<int>(32 * MB), o_slotSB = a.take<int>(32 * MB),
          o_slotLj = a.take<float2>(32 * (size_t)MB);
-  size_t o_ckey = a.take<uint32_t>(6 * (size_t)C), o_eb = a.take<int>(bnb::kExclBlk * MB),
-         o_ebc = a.take<int>(MB);
-  size_t o_cullC = a.take<int>(MB * bnb::kNumShifts), o_cullO = a.take<int>(MB * bnb::kNumShifts + 1);
-  size_t o_cand = a.take<int4>(h->capCand), o_cflag = a.take<int>(h->capCand),
-         o_cmo = a.take<int>(h->capCand + 1);
+  size_t o_ckey = a.take<uint32_t>(6 * (size_t)C);
+  size_t o_cand = a.take<int4>(h->capCand);
   size_t o_masks = a.take<uint32_t>(32 * (size_t)h->capMask);
-  size_t o_cs = a.take<int>(MB + 1), o_work = a.take<int2>(h->capWork), o_cost = a.take<unsigned int>(h->capWork),
-         o_order = a.take<int>(h->capWork);
-  size_t o_part = a.take<int>(4096);
+  const size_t W = 2 * (size_t)h->capWork;
+  size_t o_cs = a.take<int>(MB), o_cn = a.take<int>(MB), o_work = a.take<int2>(W), o_cost = a.take<unsigned int>(W),
+         o_order = a.take<int>(W);
   size_t o_xyzq = a.take<float4>(32 * MB), o_bmin = a.take<float4>(MB), o_bmax = a.take<float4>(MB);
   size_t o_hmin = a.take<float4>(2 * (size_t)MB), o_hmax = a.take<float4>(2 * (size_t)MB);
   size_t o_acc = a.take<long long>(3 * 32 * (size_t)MB);
@@ -227,7 +224,7 @@ int alloc_list(bnb_handle *h) {
   d.colCount = (int *)(b + o_cc);
   d.colStartAtom = (int *)(b + o_csa);
   d.colStartBlock = (int *)(b + o_csb);
-  d.colFill = (int *)(b + o_cf);
+  d.atomRank = (int *)(b + o_rank);
   h->colRep_d = (int *)(b + o_colrep);
   d.bucket = (int *)(b + o_bucket);
   d.sortedAtom = (int *)(b + o_sorted);
@@ -241,19 +238,13 @@ int alloc_list(bnb_handle *h) {
   d.slotSiteBlock = (int *)(b + o_slotSB);
   d.slotLj = (float2 *)(b + o_slotLj);
   d.colKey = (uint32_t *)(b + o_ckey);
-  d.exclBlk = (int *)(b + o_eb);
-  d.exclBlkCount = (int *)(b + o_ebc);
-  d.cullCount = (int *)(b + o_cullC);
-  d.cullOffset = (int *)(b + o_cullO);
   d.cand = (int4 *)(b + o_cand);
-  d.candFlag = (int *)(b + o_cflag);
-  d.candMaskOff = (int *)(b + o_cmo);
   d.masks = (uint32_t *)(b + o_masks);
   d.candStart = (int *)(b + o_cs);
+  d.candNum = (int *)(b + o_cn);
   d.work = (int2 *)(b + o_work);
   d.itemCost = (unsigned int *)(b + o_cost);
   d.order = (int *)(b + o_order);
-  d.scanPartial = (int *)(b + o_part);
   d.xyzq = (float4 *)(b + o_xyzq);
   d.bmin = (float4 *)(b + o_bmin);
   d.bmax = (float4 *)(b + o_bmax);
@@ -715,11 +706,10 @@ int bnb_rebuild(bnb_handle *h, const float *position, const float *boxes, void *
   int rc = upload_rep(h, s);
   if (rc) return rc;
   const float rcull = h->p.rCut + h->p.cullPad;
-  const float rcull2 = rcull * rcull;
   for (int attempt = 0; attempt < 12; attempt++) {
     const bool rec = h->prof && h->rebN < kProfSlots;
     if (rec) cudaEventRecord(h->rebEv[2 * h->rebN], s);
-    h->launches += bnb::rebuild_list(h->d, h->colRep_d, position, rcull2, s);
+    h->launches += bnb::rebuild_list(h->d, h->colRep_d, position, rcull, s);
     h->orderPending = true;
     if (rec) cudaEventRecord(h->rebEv[2 * h->rebN++ + 1], s);
     if (!ok(cudaGetLastError())) return BNB_ERR_CUDA;
@@ -730,6 +720,7 @@ int bnb_rebuild(bnb_handle *h, const float *position, const float *boxes, void *
     bnb::Counters c;
     if (!ok(cudaMemcpyAsync(&c, h->d.ctr, sizeof(c), cudaMemcpyDeviceToHost, s))) return BNB_ERR_CUDA;
     if (!ok(cudaStreamSynchronize(s))) return BNB_ERR_CUDA;
+    const int workCount = std::max(c.work[0], c.work[1]);  // both parts have room for capWork
     int bad = c.status & bnb::kStatusListInvalid;
     if (!bad) {
       // Keep at least 50 % headroom after a synchronous build, so that the
@@ -741,10 +732,10 @@ int bnb_rebuild(bnb_handle *h, const float *position, const float *boxes, void *
         grow = true;
       }
       if (3LL * c.maskCount > 2LL * h->capMask) { h->capMask = 2 * c.maskCount + 64; grow = true; }
-      if (3LL * c.workCount > 2LL * h->capWork) { h->capWork = 2 * c.workCount + 64; grow = true; }
+      if (3LL * workCount > 2LL * h->capWork) { h->capWork = 2 * workCount + 64; grow = true; }
       if (!grow) {
         h->listBuilt = true;
-        h->lastWork = c.workCount;
+        h->lastWork = c.work[0] + c.work[1];
         return BNB_OK;
       }
       rc = alloc_list(h);
@@ -756,19 +747,12 @@ int bnb_rebuild(bnb_handle *h, const float *position, const float *boxes, void *
     }
     if (bad & bnb::kStatusBlockOverflow) return BNB_ERR_CAPACITY;  // cannot happen by construction
     // Grow what overflowed by 1.5x (src/domdec/cull.cu:337-375) and retry.
-    int needCand = 0;
     if (bad & bnb::kStatusCandOverflow) {
-      cudaMemcpy(&needCand, h->d.cullOffset + h->maxBlocks * bnb::kNumShifts, sizeof(int),
-                 cudaMemcpyDeviceToHost);
-      h->capCand = (int)std::min<long long>((long long)std::max(needCand, h->capCand) * 3 / 2, kCapLimit);
+      h->capCand = (int)std::min<long long>((long long)std::max(c.candCount, h->capCand) * 3 / 2, kCapLimit);
       h->capWork = std::max(h->capWork, h->capCand / bnb::kMinTilesPerWork + h->maxBlocks + 16);
     }
-    if (bad & bnb::kStatusMaskOverflow) {
-      int needMask = 0;
-      cudaMemcpy(&needMask, h->d.candMaskOff + h->d.capCand, sizeof(int), cudaMemcpyDeviceToHost);
-      h->capMask = std::max(needMask, h->capMask) * 3 / 2 + 64;
-    }
-    if (bad & bnb::kStatusWorkOverflow) h->capWork = h->capWork * 3 / 2 + 64;
+    if (bad & bnb::kStatusMaskOverflow) h->capMask = std::max(c.maskCount, h->capMask) * 3 / 2 + 64;
+    if (bad & bnb::kStatusWorkOverflow) h->capWork = std::max(workCount, h->capWork) * 3 / 2 + 64;
     rc = alloc_list(h);
     if (rc) return rc;
     rc = upload_rep(h, s);
@@ -971,9 +955,9 @@ int bnb_list_sizes(bnb_handle *h, void *stream, int *blocks, int *tiles, int *ma
       !ok(cudaStreamSynchronize(s)))
     return BNB_ERR_CUDA;
   if (blocks) *blocks = c.blockCount;
-  if (tiles) *tiles = c.candCount;
-  if (masks) *masks = c.maskCount;
-  if (work) *work = c.workCount;
+  if (tiles) *tiles = std::min(c.candCount, h->capCand);
+  if (masks) *masks = std::min(c.maskCount, h->capMask);
+  if (work) *work = std::min(c.work[0], h->capWork) + std::min(c.work[1], h->capWork);
   return BNB_OK;
 }
 
@@ -1003,24 +987,35 @@ int bnb_get_list(bnb_handle *h, void *stream, int *wrap, int *blockBounds, int *
       for (int b = 0; b < B; b++) { bmax[3 * b] = t[b].x; bmax[3 * b + 1] = t[b].y; bmax[3 * b + 2] = t[b].z; }
     }
   }
-  dn(candStart, d.candStart, sizeof(int) * (B + 1));
-  if (cand || candMask) {
-    std::vector<int4> t(T > 0 ? T : 1);
+  if (candStart || cand || candMask || masks) {
+    // the device keeps the blocks' ranges in the order they were reserved and a
+    // mask word per j atom; the export is in block order with a row per i atom
+    std::vector<int> start(std::max(B, 1)), num(std::max(B, 1));
+    std::vector<int4> t(std::max(T, 1));
+    std::vector<uint32_t> words(masks ? 32 * (size_t)M : 0);
+    dn(start.data(), d.candStart, sizeof(int) * B);
+    dn(num.data(), d.candNum, sizeof(int) * B);
     dn(t.data(), d.cand, sizeof(int4) * T);
-    for (int c = 0; c < T; c++) {
-      if (cand) { cand[2 * c] = t[c].x; cand[2 * c + 1] = t[c].y; }
-      if (candMask) candMask[c] = t[c].z;
-    }
-  }
-  if (masks && M) {  // the device keeps a word per j atom; the export has a row per i atom
-    std::vector<uint32_t> t(32 * (size_t)M);
-    dn(t.data(), d.masks, sizeof(uint32_t) * t.size());
-    for (int m = 0; m < M; m++)
-      for (int i = 0; i < 32; i++) {
-        uint32_t row = 0;
-        for (int j = 0; j < 32; j++) row |= ((t[32 * (size_t)m + j] >> i) & 1u) << j;
-        masks[32 * (size_t)m + i] = row;
+    dn(words.data(), d.masks, sizeof(uint32_t) * words.size());
+    if (!good) return BNB_ERR_CUDA;
+    int at = 0, m = 0;
+    for (int i = 0; i < B; i++) {
+      if (candStart) candStart[i] = at;
+      for (int k = 0; k < num[i] && at < T; k++, at++) {
+        const int4 c = t[start[i] + k];
+        if (cand) { cand[2 * at] = c.x; cand[2 * at + 1] = c.y; }
+        if (candMask) candMask[at] = c.z < 0 ? -1 : m;
+        if (c.z < 0 || m >= M) continue;
+        if (masks)
+          for (int a = 0; a < 32; a++) {
+            uint32_t row = 0;
+            for (int j = 0; j < 32; j++) row |= ((words[32 * (size_t)c.z + j] >> a) & 1u) << j;
+            masks[32 * (size_t)m + a] = row;
+          }
+        m++;
       }
+    }
+    if (candStart) candStart[B] = at;
   }
   return good ? BNB_OK : BNB_ERR_CUDA;
 }

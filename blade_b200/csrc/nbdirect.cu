@@ -702,7 +702,8 @@ __global__ void __launch_bounds__(256, 2) k_pair(KArgs A) {
   __syncthreads();
 
   const int status = d.ctr->status;
-  const int nWork = (status & kStatusListInvalid) ? 0 : d.ctr->workCount;
+  const int nFull = d.ctr->work[0];  // full-size items; the tail items follow
+  const int nWork = (status & kStatusListInvalid) ? 0 : nFull + d.ctr->work[1];
   const int NS = 32 * d.maxBlocks;
   unsigned long long pairs = 0;
 
@@ -715,11 +716,9 @@ __global__ void __launch_bounds__(256, 2) k_pair(KArgs A) {
   while (w < nWork) {
     const int item = ordered ? d.order[w] : w;
     const long long tItem = clock64();
-    const int2 wk = d.work[item];
+    const int2 wk = d.work[item < nFull ? item : d.capWork + item - nFull];
     const int iBlock = wk.x & 0x3FFFFF;
-    const int c0 = wk.y;
-    int c1 = d.candStart[iBlock + 1];
-    c1 = c1 < c0 + (wk.x >> 22) ? c1 : c0 + (wk.x >> 22);
+    const int c0 = wk.y, c1 = c0 + (wk.x >> 22);
     const RepInfo &ri = d.rep[d.blockRep[iBlock]];
     const float4 *shifts = ri.shift;  // image shift vectors by shift code
     const float4 imin = d.bmin[iBlock], imax = d.bmax[iBlock];
@@ -890,10 +889,19 @@ __device__ __forceinline__ int cost_bucket(unsigned int c) {
 __global__ void __launch_bounds__(1024) k_order(Dev d) {
   pdl_wait();
   __shared__ int hist[256];
-  const int n = (d.ctr->status & kStatusListInvalid) ? 0 : d.ctr->workCount;
+  const int n = (d.ctr->status & kStatusListInvalid) ? 0 : d.ctr->work[0] + d.ctr->work[1];
   for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&hist[cost_bucket(d.itemCost[i])], 1);
+  // eight costs in flight per thread: the loads' latency is all it spends
+  constexpr int kBatch = 8;
+  for (int i0 = threadIdx.x; i0 < n; i0 += kBatch * blockDim.x) {
+    unsigned int c[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; k++) c[k] = i0 + k * blockDim.x < n ? d.itemCost[i0 + k * blockDim.x] : 0u;
+#pragma unroll
+    for (int k = 0; k < kBatch; k++)
+      if (i0 + k * blockDim.x < n) atomicAdd(&hist[cost_bucket(c[k])], 1);
+  }
   __syncthreads();
   if (threadIdx.x < 32) {  // lane l owns buckets 255 - 8l .. 248 - 8l (descending)
     const int l = threadIdx.x;
@@ -917,7 +925,14 @@ __global__ void __launch_bounds__(1024) k_order(Dev d) {
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) d.order[atomicAdd(&hist[cost_bucket(d.itemCost[i])], 1)] = i;
+  for (int i0 = threadIdx.x; i0 < n; i0 += kBatch * blockDim.x) {
+    unsigned int c[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; k++) c[k] = i0 + k * blockDim.x < n ? d.itemCost[i0 + k * blockDim.x] : 0u;
+#pragma unroll
+    for (int k = 0; k < kBatch; k++)
+      if (i0 + k * blockDim.x < n) d.order[atomicAdd(&hist[cost_bucket(c[k])], 1)] = i0 + k * blockDim.x;
+  }
   if (threadIdx.x == 0) d.ctr->orderValid = n > 0;
 }
 
