@@ -40,8 +40,8 @@ enum : int {
 
 // Output modes (BNB_OUT_SET / BNB_OUT_ADD64 of the public header).
 __device__ __forceinline__ void out64(double *p, double v, int mode) {
-  if (mode & BNB_OUT_ADD64) *p += v;
-  else *p = v;
+  if (!(mode & BNB_OUT_ADD64)) *p = v;
+  else if (v != 0.0) *p += v;  // most atoms have no 1-4 pair: nothing to read or write
 }
 __device__ __forceinline__ void out32(float *p, float v, int mode) {  // atomic unless overwriting
   if (mode & BNB_OUT_SET) *p = v;

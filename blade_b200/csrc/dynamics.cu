@@ -17,6 +17,10 @@
 #include <stdint.h>
 
 #include "bnb.h"
+#include "bnb_internal.h"
+
+using bnb::launch_pdl;
+using bnb::pdl_wait;
 
 namespace {
 
@@ -39,6 +43,7 @@ __global__ void k_vrorv(int nx, int nt, double *x, double *v, const double *fx, 
                         double *th, double *vt, const double *ft, const double *ismt, double dt,
                         double ax, double bx, double at, double bt, uint64_t seed, uint64_t step,
                         unsigned long long *stepCounter, float *x_f, int *nanFlag) {
+  pdl_wait();
   __shared__ bool lastBlock;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (stepCounter) step += stepCounter[0];
@@ -91,6 +96,7 @@ __global__ void k_langevin_half(int phase, int nx, int nt, double *x, double *v,
                                 const double *ismx, double *th, double *vt, const double *ft, const double *ismt,
                                 double dt, double ax, double bx, double at, double bt, uint64_t seed, uint64_t step,
                                 unsigned long long *stepCounter, float *x_f, int *nanFlag) {
+  pdl_wait();
   __shared__ bool lastBlock;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (stepCounter) step += stepCounter[0];
@@ -139,6 +145,7 @@ __global__ void k_langevin_half(int phase, int nx, int nt, double *x, double *v,
 // order fixed (no atomics) and the result reproducible bit for bit.
 __global__ void k_bonds(int n, const int *start, const int *partner, const float2 *kb_b0, const double *x,
                         double *grad) {
+  pdl_wait();
   int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
   const double xa = x[3 * a], ya = x[3 * a + 1], za = x[3 * a + 2];
@@ -164,7 +171,7 @@ extern "C" int bnb_bond_gradient(int n, const int *start, const int *partner, co
                                  const double *x, double *grad, void *stream) {
   if (n < 0 || (n > 0 && (!start || !partner || !kbB0 || !x || !grad))) return BNB_ERR_ARG;
   if (n == 0) return BNB_OK;
-  k_bonds<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(n, start, partner, (const float2 *)kbB0, x, grad);
+  launch_pdl(k_bonds, (n + 255) / 256, 256, 0, (cudaStream_t)stream, n, start, partner, (const float2 *)kbB0, x, grad);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
 
@@ -179,9 +186,8 @@ extern "C" int bnb_langevin_vrorv(int nx, int nt, double *x, double *v, const do
     return BNB_ERR_ARG;
   int n = nx + nt;
   if (n == 0) return BNB_OK;
-  k_vrorv<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(nx, nt, x, v, fx, ismx, theta, vtheta, ftheta,
-                                                             ismtheta, dt, frictionX, noiseX, frictionTheta,
-                                                             noiseTheta, seed, step, stepCounter, x_f, nanFlag);
+  launch_pdl(k_vrorv, (n + 255) / 256, 256, 0, (cudaStream_t)stream, nx, nt, x, v, fx, ismx, theta, vtheta, ftheta,
+             ismtheta, dt, frictionX, noiseX, frictionTheta, noiseTheta, seed, step, stepCounter, x_f, nanFlag);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
 
@@ -196,9 +202,8 @@ extern "C" int bnb_langevin_half(int phase, int nx, int nt, double *x, double *v
     return BNB_ERR_ARG;
   int n = nx + nt;
   if (n == 0) return BNB_OK;
-  k_langevin_half<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(phase, nx, nt, x, v, xPrev, fx, ismx, theta,
-                                                                     vtheta, ftheta, ismtheta, dt, frictionX, noiseX,
-                                                                     frictionTheta, noiseTheta, seed, step,
-                                                                     stepCounter, x_f, nanFlag);
+  launch_pdl(k_langevin_half, (n + 255) / 256, 256, 0, (cudaStream_t)stream, phase, nx, nt, x, v, xPrev, fx, ismx,
+             theta, vtheta, ftheta, ismtheta, dt, frictionX, noiseX, frictionTheta, noiseTheta, seed, step, stepCounter,
+             x_f, nanFlag);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }

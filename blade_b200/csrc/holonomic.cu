@@ -22,6 +22,10 @@
 #include <math.h>
 
 #include "bnb.h"
+#include "bnb_internal.h"
+
+using bnb::launch_pdl;
+using bnb::pdl_wait;
 
 namespace {
 
@@ -198,6 +202,7 @@ __device__ __forceinline__ Cluster<NH + 1, NH> branch(const T &t) {
 __global__ void k_holonomic_position(bnb_constraints cs, const double *xPrev, double *x, double *v,
                                      const double *ism, double halfdt, double tol, int maxIter, float *x_f,
                                      int *status) {
+  pdl_wait();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < cs.nTriangle) {
     constrain_position(triangle(cs.triangle[t]), xPrev, x, v, ism, halfdt, tol, maxIter, x_f, status);
@@ -219,6 +224,7 @@ __global__ void k_holonomic_position(bnb_constraints cs, const double *xPrev, do
 }
 
 __global__ void k_holonomic_velocity(bnb_constraints cs, const double *x, double *v, const double *ism) {
+  pdl_wait();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < cs.nTriangle) {
     constrain_velocity(triangle(cs.triangle[t]), x, v, ism);
@@ -253,8 +259,8 @@ extern "C" int bnb_holonomic_position(const bnb_constraints *cs, const double *x
     return BNB_ERR_ARG;
   const long long n = (long long)cs->nTriangle + cs->nBranch1 + cs->nBranch2 + cs->nBranch3;
   if (n == 0) return BNB_OK;
-  k_holonomic_position<<<(int)((n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(*cs, xPrev, x, v, ism, halfdt,
-                                                                                tolerance, maxIter, x_f, status);
+  launch_pdl(k_holonomic_position, (int)((n + 127) / 128), 128, 0, (cudaStream_t)stream, *cs, xPrev, x, v, ism, halfdt,
+             tolerance, maxIter, x_f, status);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
 
@@ -263,6 +269,6 @@ extern "C" int bnb_holonomic_velocity(const bnb_constraints *cs, const double *x
   if (!valid(cs) || !x || !v || !ism) return BNB_ERR_ARG;
   const long long n = (long long)cs->nTriangle + cs->nBranch1 + cs->nBranch2 + cs->nBranch3;
   if (n == 0) return BNB_OK;
-  k_holonomic_velocity<<<(int)((n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(*cs, x, v, ism);
+  launch_pdl(k_holonomic_velocity, (int)((n + 127) / 128), 128, 0, (cudaStream_t)stream, *cs, x, v, ism);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }

@@ -14,12 +14,17 @@
 #include <stdint.h>
 
 #include "bnb.h"
+#include "bnb_internal.h"
+
+using bnb::launch_pdl;
+using bnb::pdl_wait;
 
 namespace {
 
 __global__ void k_lambda_from_theta(int siteCount, const int *siteBound, double fnex,
                                     const double *theta, const uint8_t *fixed, double *lambda,
                                     float *lambda_f) {
+  pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= siteCount) return;
   int j0 = siteBound[i], j1 = siteBound[i + 1];
@@ -46,6 +51,7 @@ template <typename L, typename F>
 __global__ void k_theta_force(int blockCount, const int *lambdaSite, const int *siteBound, double fnex,
                               const L *lambda, const L *theta, const F *lambdaForce, const uint8_t *fixed,
                               F *thetaForce) {
+  pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= blockCount) return;
   if (fixed && fixed[i]) return;
@@ -69,6 +75,7 @@ __device__ void warp_energy(double e, double *energy) {
 template <typename L, typename F>
 __global__ void k_bias(int blockCount, const L *lambda, const L *fixedBias, int nVar,
                        const bnb_varbias *vb, F *lambdaForce, double *energy) {
+  pdl_wait();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   double e = 0;
   if (fixedBias && t < blockCount) {
@@ -115,6 +122,7 @@ __global__ void k_bias(int blockCount, const L *lambda, const L *fixedBias, int 
 __global__ void k_lambda_histogram(int blockCount, const double *lambda, const uint8_t *fixed, int pairCount,
                                    const int *pairs, unsigned int *hist1, unsigned int *hist2,
                                    unsigned int *endCount) {
+  pdl_wait();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < blockCount && !(fixed && fixed[t])) {
     const double l = lambda[t];
@@ -141,8 +149,9 @@ int theta_force(int blockCount, const int *lambdaSite, const int *siteBound, dou
                                             !lambdaForce || !thetaForce)))
     return BNB_ERR_ARG;
   if (blockCount == 0) return BNB_OK;
-  k_theta_force<L, F><<<blocks_for(blockCount), 256, 0, (cudaStream_t)stream>>>(
-      blockCount, lambdaSite, siteBound, fnex, lambda, theta, lambdaForce, blockFixed, thetaForce);
+  auto kernel = k_theta_force<L, F>;
+  launch_pdl(kernel, blocks_for(blockCount), 256, 0, (cudaStream_t)stream, blockCount, lambdaSite, siteBound,
+             fnex, lambda, theta, lambdaForce, blockFixed, thetaForce);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
 
@@ -153,8 +162,9 @@ int bias(int blockCount, const L *lambda, const L *fixedBias, int varCount, cons
     return BNB_ERR_ARG;
   int n = blockCount > varCount ? blockCount : varCount;
   if (n == 0) return BNB_OK;
-  k_bias<L, F><<<blocks_for(n), 256, 0, (cudaStream_t)stream>>>(blockCount, lambda, fixedBias, varCount,
-                                                                varBias, lambdaForce, energy);
+  auto biasKernel = k_bias<L, F>;
+  launch_pdl(biasKernel, blocks_for(n), 256, 0, (cudaStream_t)stream, blockCount, lambda, fixedBias, varCount,
+             varBias, lambdaForce, energy);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
 
@@ -165,8 +175,7 @@ extern "C" int bnb_lambda_from_theta(int siteCount, const int *siteBound, double
                                      float *lambda_f, void *stream) {
   if (siteCount < 0 || (siteCount > 0 && (!siteBound || !theta || !lambda))) return BNB_ERR_ARG;
   if (siteCount == 0) return BNB_OK;
-  k_lambda_from_theta<<<blocks_for(siteCount), 256, 0, (cudaStream_t)stream>>>(
-      siteCount, siteBound, fnex, theta, blockFixed, lambda, lambda_f);
+  launch_pdl(k_lambda_from_theta, blocks_for(siteCount), 256, 0, (cudaStream_t)stream, siteCount, siteBound, fnex, theta, blockFixed, lambda, lambda_f);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
 
@@ -202,7 +211,7 @@ extern "C" int bnb_lambda_histogram(int blockCount, const double *lambda, const 
     return BNB_ERR_ARG;
   const int n = blockCount > pairCount ? blockCount : pairCount;
   if (n == 0) return BNB_OK;
-  k_lambda_histogram<<<blocks_for(n), 256, 0, (cudaStream_t)stream>>>(blockCount, lambda, blockFixed, pairCount,
+  launch_pdl(k_lambda_histogram, blocks_for(n), 256, 0, (cudaStream_t)stream, blockCount, lambda, blockFixed, pairCount,
                                                                       pairs, hist1, hist2, endCount);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }

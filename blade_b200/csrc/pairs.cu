@@ -130,6 +130,7 @@ __device__ __forceinline__ void apply(const PairsArgs &a, int ii, int jj, const 
 
 template <int ELEC, int VDW, bool SOFT, bool ENERGY>
 __global__ void k_nb14(PairsArgs a) {
+  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.n14) return;
   const bnb_nb14 pp = a.nb14[t];
@@ -160,6 +161,7 @@ __global__ void k_nb14(PairsArgs a) {
 
 template <bool ENERGY>
 __global__ void k_nbex(PairsArgs a) {
+  pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= a.nex) return;
   const bnb_nbex pp = a.nbex[t];
@@ -180,6 +182,7 @@ __global__ void k_nbex(PairsArgs a) {
 }
 
 __global__ void k_pairs_finalize(PairsArgs a, bnb_outputs o) {
+  pdl_wait();
   const double inv = 1.0 / kFixScale;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * a.N; t += gridDim.x * blockDim.x) {
     const long long v = a.accF[t];
@@ -209,18 +212,18 @@ __global__ void k_pairs_finalize(PairsArgs a, bnb_outputs o) {
 template <int ELEC, int VDW>
 void nb14_ev(const PairsArgs &a, bool soft, bool energy, int grid, cudaStream_t s) {
   if (soft) {
-    if (energy) k_nb14<ELEC, VDW, true, true><<<grid, 256, 0, s>>>(a);
-    else k_nb14<ELEC, VDW, true, false><<<grid, 256, 0, s>>>(a);
+    if (energy) launch_pdl(k_nb14<ELEC, VDW, true, true>, grid, 256, 0, s, a);
+    else launch_pdl(k_nb14<ELEC, VDW, true, false>, grid, 256, 0, s, a);
   } else {
-    if (energy) k_nb14<ELEC, VDW, false, true><<<grid, 256, 0, s>>>(a);
-    else k_nb14<ELEC, VDW, false, false><<<grid, 256, 0, s>>>(a);
+    if (energy) launch_pdl(k_nb14<ELEC, VDW, false, true>, grid, 256, 0, s, a);
+    else launch_pdl(k_nb14<ELEC, VDW, false, false>, grid, 256, 0, s, a);
   }
 }
 
 void finalize(const PairsArgs &a, const bnb_outputs &o, cudaStream_t s) {
   int grid = (3 * a.N + 255) / 256;
   grid = grid < 1 ? 1 : (grid > 148 * 8 ? 148 * 8 : grid);
-  k_pairs_finalize<<<grid, 256, 0, s>>>(a, o);
+  launch_pdl(k_pairs_finalize, grid, 256, 0, s, a, o);
 }
 
 }  // namespace
@@ -250,8 +253,8 @@ int launch_nb14(const PairsArgs &a, const bnb_outputs &o, int elec, int vdw, boo
 int launch_nbex(const PairsArgs &a, const bnb_outputs &o, bool energy, cudaStream_t s) {
   if (a.nex > 0) {
     const int grid = (a.nex + 255) / 256;
-    if (energy) k_nbex<true><<<grid, 256, 0, s>>>(a);
-    else k_nbex<false><<<grid, 256, 0, s>>>(a);
+    if (energy) launch_pdl(k_nbex<true>, grid, 256, 0, s, a);
+    else launch_pdl(k_nbex<false>, grid, 256, 0, s, a);
     if (cudaGetLastError() != cudaSuccess) return BNB_ERR_CUDA;
   }
   finalize(a, o, s);
