@@ -3,7 +3,7 @@
 // Counterparts of Msld::calc_lambda_from_theta (src/msld/msld.cu:863-921),
 // Msld::calc_thetaForce_from_lambdaForce (msld.cu:937-998) and the fixed and
 // variable lambda biases (msld.cu:1000-1153).  These are tiny per-site /
-// per-block / per-bias loops: one thread each.  Entry points come in the
+// per-block / per-bias loops: a warp or a thread each.  Entry points come in the
 // FP64 form and, for the buffers BLaDE's State keeps in FP32 (lambda_fd,
 // theta_fd, lambdaForce_d, thetaForce_d, lambdaBias_d), an FP32-buffer form
 // that still computes in FP64.  Block-fixed flags are byte arrays, the
@@ -25,22 +25,30 @@ __global__ void k_lambda_from_theta(int siteCount, const int *siteBound, double 
                                     const double *theta, const uint8_t *fixed, double *lambda,
                                     float *lambda_f) {
   pdl_wait();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  // a warp per site: exp(sin()) of its blocks side by side, summed in block order
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= siteCount) return;
-  int j0 = siteBound[i], j1 = siteBound[i + 1];
+  const int j0 = siteBound[i], j1 = siteBound[i + 1];
   double fixsum = 0, norm = 0;
-  for (int j = j0; j < j1; j++) {
-    if (fixed && fixed[j]) {
-      fixsum += theta[j];
-    } else {
-      double l = exp(fnex * sin(theta[j]));
-      lambda[j] = l;
-      norm += l;
+  for (int c = j0; c < j1; c += 32) {
+    const int j = c + lane, n = j1 - c < 32 ? j1 - c : 32;
+    double l = 0;
+    bool fx = false;
+    if (j < j1) {
+      fx = fixed && fixed[j];
+      l = fx ? theta[j] : exp(fnex * sin(theta[j]));
+      if (!fx) lambda[j] = l;
+    }
+    const unsigned mask = __ballot_sync(0xFFFFFFFFu, fx);
+    for (int k = 0; k < n; k++) {
+      const double v = __shfl_sync(0xFFFFFFFFu, l, k);
+      if (mask >> k & 1u) fixsum += v;
+      else norm += v;
     }
   }
   double rfrac = 1.0 - fixsum;
   if (norm > 0) norm = rfrac / norm;
-  for (int j = j0; j < j1; j++) {
+  for (int j = j0 + lane; j < j1; j += 32) {  // each lane reads back what it wrote
     double l = (fixed && fixed[j]) ? theta[j] : lambda[j] * norm;
     lambda[j] = l;
     if (lambda_f) lambda_f[j] = (float)l;
@@ -140,7 +148,7 @@ __global__ void k_lambda_histogram(int blockCount, const double *lambda, const u
   }
 }
 
-inline int blocks_for(int n) { return n > 0 ? (n + 255) / 256 : 1; }
+inline int blocks_for(long long n) { return n > 0 ? (int)((n + 255) / 256) : 1; }
 
 template <typename L, typename F>
 int theta_force(int blockCount, const int *lambdaSite, const int *siteBound, double fnex, const L *lambda,
@@ -175,7 +183,7 @@ extern "C" int bnb_lambda_from_theta(int siteCount, const int *siteBound, double
                                      float *lambda_f, void *stream) {
   if (siteCount < 0 || (siteCount > 0 && (!siteBound || !theta || !lambda))) return BNB_ERR_ARG;
   if (siteCount == 0) return BNB_OK;
-  launch_pdl(k_lambda_from_theta, blocks_for(siteCount), 256, 0, (cudaStream_t)stream, siteCount, siteBound, fnex, theta, blockFixed, lambda, lambda_f);
+  launch_pdl(k_lambda_from_theta, blocks_for(32ll * siteCount), 256, 0, (cudaStream_t)stream, siteCount, siteBound, fnex, theta, blockFixed, lambda, lambda_f);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
 

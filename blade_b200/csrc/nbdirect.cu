@@ -670,12 +670,17 @@ struct WarpSmem<COMBINE, 0> {
   Queue<COMBINE, false, queue_places<0>()> plain;
 };
 
+// Resident warps, at 128 registers: 16 in 2 CTAs.  18 warps (3 x 6, 112
+// registers) and 20 (4 x 5, 96) spill: chain of 23,558 atoms 697 -> 724 and 738 us a
+// ten-step pass, 32 MSLD boxes 1025 -> 1113 and 1163; 4 CTAs of 4 the same as 2 of 8.
+constexpr int kPairWarps = 8, kPairCtas = 2;
+
 // ---------------------------------------------------------------------------
 // The pair kernel.
 // ALCH: 0 none, 1 MSLD scaling, 2 MSLD scaling + soft core.
 // ---------------------------------------------------------------------------
 template <int ELEC, int VDW, int ALCH, bool ENERGY, bool COMBINE>
-__global__ void __launch_bounds__(256, 2) k_pair(KArgs A) {
+__global__ void __launch_bounds__(32 * kPairWarps, kPairCtas) k_pair(KArgs A) {
   pdl_wait();
   extern __shared__ __align__(16) unsigned char smem[];
   const Dev &d = A.d;
@@ -684,8 +689,8 @@ __global__ void __launch_bounds__(256, 2) k_pair(KArgs A) {
   const int nT = d.nTypes;
   using Warp = WarpSmem<COMBINE, ALCH>;
   Warp &ws = reinterpret_cast<Warp *>(smem)[threadIdx.x >> 5];
-  float2 *sLJ = reinterpret_cast<float2 *>(smem + 8 * sizeof(Warp));
-  const size_t off = 8 * sizeof(Warp) + (COMBINE ? 0 : (sizeof(float2) * nT * nT + 15) & ~size_t(15));
+  float2 *sLJ = reinterpret_cast<float2 *>(smem + kPairWarps * sizeof(Warp));
+  const size_t off = kPairWarps * sizeof(Warp) + (COMBINE ? 0 : (sizeof(float2) * nT * nT + 15) & ~size_t(15));
   long long *sAccL = reinterpret_cast<long long *>(smem + off);
   float *sLam = reinterpret_cast<float *>(smem + off + (ALCH ? sizeof(long long) * d.lamTotal : 0));
 
@@ -979,7 +984,7 @@ __global__ void k_finalize(Dev d, bnb_outputs o, int mode) {
 template <int ELEC, int VDW, int ALCH, bool ENERGY, bool COMBINE>
 void launch_t(const KArgs &a, int maxGrid, size_t shmem, cudaStream_t s) {
   auto k = k_pair<ELEC, VDW, ALCH, ENERGY, COMBINE>;
-  shmem += 8 * sizeof(WarpSmem<COMBINE, ALCH>);
+  shmem += kPairWarps * sizeof(WarpSmem<COMBINE, ALCH>);
   static int perSM = -1, sms = 0;
   static size_t shmemSeen = ~size_t(0);
   if (shmem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);
@@ -987,14 +992,14 @@ void launch_t(const KArgs &a, int maxGrid, size_t shmem, cudaStream_t s) {
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, 256, shmem) != cudaSuccess || perSM < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, 32 * kPairWarps, shmem) != cudaSuccess || perSM < 1)
       perSM = 1;
     shmemSeen = shmem;
   }
   int grid = perSM * sms;
   if (grid > maxGrid) grid = maxGrid;
   if (grid < 1) grid = 1;
-  launch_pdl(k, grid, 256, shmem, s, a);
+  launch_pdl(k, grid, 32 * kPairWarps, shmem, s, a);
 }
 
 template <int ELEC, int VDW>
