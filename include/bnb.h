@@ -255,7 +255,8 @@ int bnb_compute_nbex(bnb_handle *h, const float *position, const float *lambda,
  * PME reciprocal space and the Ewald self term (getforce_ewald and
  * getforce_ewaldself, src/nbrecip/nbrecip.cu:19-555; grids and B-spline
  * moduli as Potential::initialize, src/system/potential.cxx:1202-1300).
- * bnb_set_pme sizes one grid per replica and makes the cuFFT plans:
+ * bnb_set_pme sizes one grid per replica and makes the tables of the own
+ * transforms (cuFFT plans for grids outside their range):
  *   order    B-spline order 4, 6 or 8 (Run::orderEwald, default 6)
  *   gridSpace, grid  host int [3*replicas] grid sizes, or NULL for the
  *            reference's rule from the spacing (Run::gridSpace, default 1 A):

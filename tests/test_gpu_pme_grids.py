@@ -60,3 +60,21 @@ def test_mixed_sizes_in_one_handle(cuda):
         assert np.array_equal(f[nb.starts[r]:nb.starts[r + 1]], f1) and e[r] == e1[0]
         one.close()
     nb.close()
+
+
+@pytest.mark.parametrize("order", [4, 6, 8])
+@pytest.mark.parametrize("side,box", [(1, 12.0), (2, 12.0), (15, 47.14), (16, 50.28)])
+def test_sizes_of_the_spread_and_gather(cuda, order, side, box):
+    """A few atoms, and both sides of the line between small and large warps' shares (10,656 and 9,472 atoms)."""
+    s = systems.water_box(9, n_side=side, box=box, rCut=6.0, rSwitch=5.0)
+    if side == 16:
+        s = dataclasses.replace(s, xyz=s.xyz[:-2], nbonds=s.nbonds[:-2], excl=s.excl[(s.excl < s.N - 2).all(1)])
+    nb = NbDirect(s)
+    nb.set_pme(order, grid=[(32, 32, 32)])
+    f, _, e = _run(nb)
+    eo, go, _, _ = pme_oracle.pme_recip(s.xyz, s.nbonds["q"], s.box, (32, 32, 32), order,
+                                        float(np.float32(s.betaEwald)), float(np.float32(systems.KELEC_AKMA)))
+    nb.close()
+    # FP32 grid values: relative to the scale of the largest terms, which cancel in few waters
+    assert np.sqrt(((f - go) ** 2).sum()) <= 2e-5 * max(np.sqrt((go ** 2).sum()), 1e-2)
+    assert abs(e[0] - eo) <= 2e-5 * max(abs(eo), s.N)
