@@ -362,15 +362,17 @@ struct TileFetch {
 // MSLD pairs (ALCH) have queues of their own: every j atom of an i block with
 // MSLD atoms, and MSLD j atoms of other blocks.
 // ---------------------------------------------------------------------------
-// Places of a queue.  A round is due when both halves have 32 entries, or when
-// one half could overflow with the next tile, so the halves may differ by up to
-// PLACES - 64 entries before a round runs half empty.
-// Measured: 64 places 0.5-1 % slower than 96 without MSLD, 128 no faster; with
-// MSLD, 96 places leave too little L1 (batch of 32 small boxes 90 us against 76).
-template <int ALCH>
-constexpr int queue_places() {
-  return ALCH ? 64 : 96;
-}
+// Places of the two queues.  A round is due when both halves have 32 entries, or
+// when one half could overflow with the next tile, so the halves may differ by up
+// to places - 64 entries before a round runs half empty.  The number decides which
+// entries share a round, and with it the order of the FP32 sums, so it is the same
+// in every kernel: a replica without MSLD atoms gives the same bits in a batch with
+// MSLD replicas as alone.
+// Measured: plain, 64 places are 0.5-1 % slower than 96, 128 no faster; MSLD, 96
+// leave too little L1 (batch of 32 small boxes 90 us against 76).  96 instead of
+// 64 plain places beside the MSLD queue cost no more than 1 % (32 MSLD boxes 55.8
+// against 55.4 us a force evaluation, 8 solvated replicas 178 us either way).
+constexpr int kPlainPlaces = 96, kMsldPlaces = 64;
 
 template <bool COMBINE, bool MSLD, int PLACES>
 struct Queue {
@@ -662,12 +664,12 @@ __device__ __forceinline__ void run_round(const Dev &d, const PairConst &pc, con
 // Per-warp shared memory of k_pair.
 template <bool COMBINE, int ALCH>
 struct WarpSmem {
-  Queue<COMBINE, false, queue_places<ALCH>()> plain;
-  Queue<COMBINE, true, queue_places<ALCH>()> msld;
+  Queue<COMBINE, false, kPlainPlaces> plain;
+  Queue<COMBINE, true, kMsldPlaces> msld;
 };
 template <bool COMBINE>
 struct WarpSmem<COMBINE, 0> {
-  Queue<COMBINE, false, queue_places<0>()> plain;
+  Queue<COMBINE, false, kPlainPlaces> plain;
 };
 
 // Resident warps, at 128 registers: 16 in 2 CTAs.  18 warps (3 x 6, 112
@@ -773,7 +775,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairCtas) k_pair(KArgs A) {
 #pragma unroll
     for (int h = 0; h < 2; h++) fx[h] = fy[h] = fz[h] = f2(0.f);
     long long ei = 0;  // fixed-point energy of this lane's pairs
-    Fill<queue_places<ALCH>()> plain, msld;
+    Fill<kPlainPlaces> plain;
+    Fill<kMsldPlaces> msld;
 
     // The loads of each tile are issued one tile ahead, so their latency
     // overlaps the rounds and the queueing of the tile before.

@@ -93,3 +93,41 @@ def test_default_split_follows_the_replica_and_keeps_the_list(cuda):
         assert torch.equal(f[nb.starts[r]:nb.starts[r + 1]], one.evaluate(p)[0])
         one.close()
     nb.close()
+
+
+def _msld_of_waters(seed):
+    """A water box whose first six molecules are the blocks of two sites (few
+    types, so the LJ table is in shared memory alone and in a batch)."""
+    s = systems.water_box(seed)
+    s.msld = systems._msld_layout(np.random.default_rng(seed), [3, 3])
+    s.nbonds = s.nbonds.copy()
+    for b in range(1, 7):
+        s.nbonds["siteBlock"][3 * (b - 1):3 * b] = (int(s.msld.lambdaSite[b]) << 16) | b
+    return s
+
+
+@pytest.mark.parametrize("methods", [(1, 0)])
+@pytest.mark.parametrize("n_side", [6, 16])
+def test_water_beside_msld_replica_keeps_its_bits(cuda, n_side, methods):
+    """The kernel of a batch with MSLD replicas sums a replica without MSLD
+    atoms in the order of the kernel that it runs in alone."""
+    water = systems.water_box(5, n_side=n_side, box=n_side * 18.856 / 6)
+    pair = [water, _msld_of_waters(9)]
+    for s in pair:
+        s.elecMethod, s.vdwMethod = methods
+    nb = NbDirect(pair)
+    pos, lam = nb.positions_tensor(), nb.lambdas_tensor()
+    nb.update_domdec(pos, True)
+    f, l, e = nb.evaluate(pos, lam)
+    f1 = nb.evaluate(pos, lam, calc_energy=False)[0]
+    for r, s in enumerate(pair):
+        one = NbDirect(s)
+        p = one.positions_tensor()
+        one.update_domdec(p, True)
+        g, m, d = one.evaluate(p)
+        at = slice(nb.starts[r], nb.starts[r + 1])
+        assert torch.equal(f[at], g) and float(e[r]) == float(d[0])
+        assert torch.equal(f1[at], one.evaluate(p, calc_energy=False)[0])
+        assert torch.equal(l[nb.lam_starts[r]:nb.lam_starts[r + 1]], m)
+        one.close()
+    nb.close()
