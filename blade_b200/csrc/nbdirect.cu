@@ -115,6 +115,9 @@ __device__ __forceinline__ void red_add(long long *p, long long v) {
 // ---------------------------------------------------------------------------
 // Pair physics at distance r (rinv = 1/r, r2 = r*r): energy E and dE/dr.
 // Electrostatics: nbdirect.cu:281-323; van der Waals: nbdirect.cu:326-396.
+// Every sum says whether it is fused: left to the compiler, that differs between
+// the kernels that inline this (with and without energy, MSLD, masks), and a
+// replica would not have the same bits in a batch with MSLD replicas as alone.
 // ---------------------------------------------------------------------------
 template <int ELEC, int VDW, bool NEEDE>
 __device__ __forceinline__ void pair_terms(const PairConst &pc, float r, float r2, float rinv,
@@ -131,7 +134,7 @@ __device__ __forceinline__ void pair_terms(const PairConst &pc, float r, float r
   } else if (ELEC == 0) {  // FSWITCH
     if (r <= pc.rswitch) {
       fe = -qq * rinv * rinv;
-      if (NEEDE) ee = qq * (rinv + pc.fdvc);
+      if (NEEDE) ee = qq * __fadd_rn(rinv, pc.fdvc);
     } else {
       // The reference's expanded polynomial (nbdirect.cu:293-299) cancels to
       // ~0 near rCut; in FP32 that costs ~1e-5 relative force error.  The same
@@ -139,54 +142,56 @@ __device__ __forceinline__ void pair_terms(const PairConst &pc, float r, float r
       //   dE/dr = -qq (rc^2-r^2)^2 (rc^2+2r^2-3rs^2) ginv / r^2
       //   E     =  qq (rc-r)^3 P(r) ginv / (5 r),
       //   P(r)  = 2r^3 + 6 rc r^2 + (7rc^2-5rs^2) r + 5rc^3 - 15 rc rs^2.
-      float w = pc.roff2 - r2;
+      float w = __fsub_rn(pc.roff2, r2);
       fe = -qq * (w * w * fmaf(2.f, r2, pc.fsC1) * pc.fsG) * (rinv * rinv);
       if (NEEDE) {
-        float t = pc.rcut - r;
+        float t = __fsub_rn(pc.rcut, r);
         float p = fmaf(fmaf(fmaf(2.f, r, pc.fsP1), r, pc.fsP2), r, pc.fsP3);
         ee = qq * (t * t * t) * p * pc.fsG5 * rinv;
       }
     }
   } else {  // FSHIFT
     float ri2 = pc.rcinv * pc.rcinv;
-    fe = -qq * (rinv * rinv - ri2);
-    if (NEEDE) ee = qq * (rinv - 2.f * pc.rcinv + r * ri2);
+    fe = -qq * fmaf(rinv, rinv, -ri2);
+    if (NEEDE) ee = qq * fmaf(r, ri2, fmaf(-2.f, pc.rcinv, rinv));
   }
   float rinv2 = rinv * rinv;
   float rinv3 = rinv2 * rinv;
   float rinv6 = rinv3 * rinv3;
-  float fl, el = 0.f;
+  float el = 0.f;
   if (VDW == 0) {  // VFSWITCH, branch free
     bool in = r < pc.rswitch;
-    float a = in ? rinv3 : pc.k6 * (rinv3 - pc.rci3);
-    float b = in ? rinv6 : pc.k12 * (rinv6 - pc.rci6);
-    fl = (6.f * c6 * a * rinv3 - 12.f * c12 * b * rinv6) * rinv;
+    float d3 = fmaf(rinv2, rinv, -pc.rci3), d6 = fmaf(rinv3, rinv3, -pc.rci6);
+    float a = in ? rinv3 : pc.k6 * d3;
+    float b = in ? rinv6 : pc.k12 * d6;
+    dEdr = fmaf(fmaf(6.f * c6 * a, rinv3, -(12.f * c12 * b * rinv6)), rinv, fe);
     if (NEEDE) {
-      float pe = in ? fmaf(rinv6, rinv6, -pc.dv12) : b * (rinv6 - pc.rci6);
-      float qe = in ? rinv6 - pc.dv6 : a * (rinv3 - pc.rci3);
-      el = c12 * pe - c6 * qe;
+      float pe = in ? fmaf(rinv6, rinv6, -pc.dv12) : b * d6;
+      float qe = in ? fmaf(rinv3, rinv3, -pc.dv6) : a * d3;
+      el = fmaf(c12, pe, -(c6 * qe));
     }
   } else if (VDW == 1) {  // VSWITCH
+    float f = fmaf(-12.f * c12, rinv6, 6.f * c6), e = fmaf(c12, rinv6, -c6);
     if (r < pc.rswitch) {
-      fl = (6.f * c6 - 12.f * c12 * rinv6) * rinv6 * rinv;
-      if (NEEDE) el = (c12 * rinv6 - c6) * rinv6;
+      dEdr = fmaf(f * rinv6, rinv, fe);
+      if (NEEDE) el = e * rinv6;
     } else {
-      float rijl = pc.ron2 - r2, riju = pc.roff2 - r2;
-      float fsw = riju * riju * (riju - 3.f * rijl) * pc.rul3inv;
+      float rijl = __fsub_rn(pc.ron2, r2), riju = __fsub_rn(pc.roff2, r2);
+      float fsw = riju * riju * fmaf(-3.f, rijl, riju) * pc.rul3inv;
       float dfsw = rijl * riju * pc.rul12;
-      fl = fsw * (6.f * c6 - 12.f * c12 * rinv6) * rinv6 * rinv + dfsw * (c12 * rinv6 - c6) * rinv6;
-      if (NEEDE) el = fsw * (c12 * rinv6 - c6) * rinv6;
+      dEdr = fmaf(fsw * f * rinv6, rinv, fmaf(dfsw * e, rinv6, fe));
+      if (NEEDE) el = fsw * e * rinv6;
     }
   } else {  // VSHIFT
     float r5 = r2 * r2 * r, r6 = r2 * r2 * r2;
     float rinv12 = rinv6 * rinv6;
-    fl = 6.f * c6 * (rinv6 * rinv - r5 * pc.vshRc12inv) - 12.f * c12 * (rinv12 * rinv + r5 * pc.vshRc18inv);
+    dEdr = fmaf(6.f * c6, fmaf(rinv6, rinv, -(r5 * pc.vshRc12inv)),
+                fmaf(-12.f * c12, fmaf(rinv12, rinv, r5 * pc.vshRc18inv), fe));
     if (NEEDE)
-      el = c12 * (rinv12 + 2.f * r6 * pc.vshRc18inv - 3.f * pc.vshRc12inv) -
-           c6 * (rinv6 + r6 * pc.vshRc12inv - 2.f * pc.vshRc6inv);
+      el = fmaf(c12, fmaf(-3.f, pc.vshRc12inv, fmaf(2.f * r6, pc.vshRc18inv, rinv12)),
+                -(c6 * fmaf(-2.f, pc.vshRc6inv, fmaf(r6, pc.vshRc12inv, rinv6))));
   }
-  dEdr = fe + fl;
-  E = ee + el;
+  E = __fadd_rn(ee, el);
 }
 
 // LJ pair coefficients.  Combination mode stores per type (sqrt(12 eps),

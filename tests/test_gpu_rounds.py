@@ -106,7 +106,7 @@ def _msld_of_waters(seed):
     return s
 
 
-@pytest.mark.parametrize("methods", [(1, 0)])
+@pytest.mark.parametrize("methods", [(e, v) for e in range(3) for v in range(3)])
 @pytest.mark.parametrize("n_side", [6, 16])
 def test_water_beside_msld_replica_keeps_its_bits(cuda, n_side, methods):
     """The kernel of a batch with MSLD replicas sums a replica without MSLD
