@@ -55,6 +55,7 @@ struct bnb_handle {
   int tailItems = 0;
   bool tuned = false;  // the caller's tuning; until then every replica has its own (replica_tiles)
   int smCount = 0;
+  int pairCtas[2] = {0, 0};  // resident CTAs per SM of the pair kernel without and with energy (0: not asked)
   bool counting = false;
   bool orderPending = false;  // sort the work items by cost after the next pair launch
   // profiling (bnb_profile)
@@ -648,6 +649,7 @@ int bnb_set_topology(bnb_handle *h, const bnb_nbond *nbonds, const int *typeCoun
   up(d.exclAtom, exAtom.data(), sizeof(int) * exAtom.size());
   if (!good) return BNB_ERR_CUDA;
   h->repDev.clear();  // new device table: upload on the next rebuild
+  h->pairCtas[0] = h->pairCtas[1] = 0;
   h->topo = true;
   free_list(h);  // any previous list refers to the old topology
   for (auto &r : h->rep) { r.divX = -1; r.divY = -1; r.colStart = -1; }
@@ -787,7 +789,7 @@ int bnb_compute(bnb_handle *h, const float *position, const float *lambda, const
   const bool rec = h->prof && h->pairN < kProfSlots;
   if (rec) cudaEventRecord(h->pairEv[2 * h->pairN], s);
   int rc = bnb::launch_pair(h->d, h->pc, lambda, h->p.elecMethod, h->p.vdwMethod, alch,
-                            (calcEnergy & 1) != 0, h->counting, grid, s);
+                            (calcEnergy & 1) != 0, h->counting, grid, h->smCount, h->pairCtas[calcEnergy & 1], s);
   if (rec) cudaEventRecord(h->pairEv[2 * h->pairN++ + 1], s);
   if (rc) return rc;
   bnb::launch_finalize(h->d, *out, out_mode(calcEnergy), s);

@@ -988,33 +988,36 @@ __global__ void k_finalize(Dev d, bnb_outputs o, int mode) {
 }
 
 // Persistent launch: as many CTAs as fit at once; warps pull work items from
-// the device counter, so the grid never leaves a partial last wave.
+// the device counter, so the grid never leaves a partial last wave.  `resident`
+// is the handle's own (CTAs an SM holds of this kernel at its size, 0 until
+// asked for).  The shared-memory limit belongs to the kernel, which all handles
+// and threads share: it is set to the most that any handle may ask for, so no
+// call takes another's setting back.
 template <int ELEC, int VDW, int ALCH, bool ENERGY, bool COMBINE>
-void launch_t(const KArgs &a, int maxGrid, size_t shmem, cudaStream_t s) {
+void launch_t(const KArgs &a, int maxGrid, int sms, int &resident, size_t shmem, cudaStream_t s) {
   auto k = k_pair<ELEC, VDW, ALCH, ENERGY, COMBINE>;
-  shmem += kPairWarps * sizeof(WarpSmem<COMBINE, ALCH>);
-  static int perSM = -1, sms = 0;
-  static size_t shmemSeen = ~size_t(0);
-  if (shmem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem);
-  if (perSM < 0 || shmemSeen != shmem) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, 32 * kPairWarps, shmem) != cudaSuccess || perSM < 1)
-      perSM = 1;
-    shmemSeen = shmem;
+  constexpr size_t queues = kPairWarps * sizeof(WarpSmem<COMBINE, ALCH>);
+  constexpr size_t most = queues + (COMBINE ? 0 : sizeof(float2) * kMaxTableTypes * kMaxTableTypes) +
+                          (ALCH ? (sizeof(long long) + sizeof(float)) * kMaxLambdaShared : 0);
+  static_assert(most <= 227 * 1024, "fits an SM");
+  shmem += queues;
+  if (resident == 0) {
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k, 32 * kPairWarps, shmem) != cudaSuccess ||
+        resident < 1)
+      resident = 1;
   }
-  int grid = perSM * sms;
+  int grid = resident * sms;
   if (grid > maxGrid) grid = maxGrid;
   if (grid < 1) grid = 1;
   launch_pdl(k, grid, 32 * kPairWarps, shmem, s, a);
 }
 
 template <int ELEC, int VDW>
-void launch_ev(const KArgs &a, int alch, bool energy, bool combine, int grid, size_t shmem,
+void launch_ev(const KArgs &a, int alch, bool energy, bool combine, int grid, int sms, int &resident, size_t shmem,
                cudaStream_t s) {
 #define BNB_L(AL, EN, CO) \
-  if (alch == AL && energy == EN && combine == CO) { launch_t<ELEC, VDW, AL, EN, CO>(a, grid, shmem, s); return; }
+  if (alch == AL && energy == EN && combine == CO) { launch_t<ELEC, VDW, AL, EN, CO>(a, grid, sms, resident, shmem, s); return; }
   BNB_L(0, false, false) BNB_L(0, false, true) BNB_L(0, true, false) BNB_L(0, true, true)
   BNB_L(1, false, false) BNB_L(1, false, true) BNB_L(1, true, false) BNB_L(1, true, true)
   BNB_L(2, false, false) BNB_L(2, false, true) BNB_L(2, true, false) BNB_L(2, true, true)
@@ -1154,7 +1157,7 @@ void launch_allpairs_ev(const AllPairsArgs &a, bool energy, dim3 grid, cudaStrea
 }  // namespace
 
 int launch_pair(const Dev &d, const PairConst &pc, const float *lambda, int elec, int vdw,
-                int alch, bool energy, bool count, int grid, cudaStream_t s) {
+                int alch, bool energy, bool count, int grid, int sms, int &resident, cudaStream_t s) {
   if (32LL * d.maxBlocks >= (1LL << 27)) return BNB_ERR_TOO_LARGE;  // streamed entries hold the slot in 27 bits
   KArgs a{d, pc, lambda, count ? 1 : 0};
   size_t shmem = d.ljCombine ? 0 : sizeof(float2) * d.nTypes * d.nTypes;
@@ -1162,15 +1165,15 @@ int launch_pair(const Dev &d, const PairConst &pc, const float *lambda, int elec
   if (alch) shmem += (sizeof(long long) + sizeof(float)) * d.lamTotal;
   bool combine = d.ljCombine != 0;
   switch (elec * 3 + vdw) {
-    case 0: launch_ev<0, 0>(a, alch, energy, combine, grid, shmem, s); break;
-    case 1: launch_ev<0, 1>(a, alch, energy, combine, grid, shmem, s); break;
-    case 2: launch_ev<0, 2>(a, alch, energy, combine, grid, shmem, s); break;
-    case 3: launch_ev<1, 0>(a, alch, energy, combine, grid, shmem, s); break;
-    case 4: launch_ev<1, 1>(a, alch, energy, combine, grid, shmem, s); break;
-    case 5: launch_ev<1, 2>(a, alch, energy, combine, grid, shmem, s); break;
-    case 6: launch_ev<2, 0>(a, alch, energy, combine, grid, shmem, s); break;
-    case 7: launch_ev<2, 1>(a, alch, energy, combine, grid, shmem, s); break;
-    case 8: launch_ev<2, 2>(a, alch, energy, combine, grid, shmem, s); break;
+    case 0: launch_ev<0, 0>(a, alch, energy, combine, grid, sms, resident, shmem, s); break;
+    case 1: launch_ev<0, 1>(a, alch, energy, combine, grid, sms, resident, shmem, s); break;
+    case 2: launch_ev<0, 2>(a, alch, energy, combine, grid, sms, resident, shmem, s); break;
+    case 3: launch_ev<1, 0>(a, alch, energy, combine, grid, sms, resident, shmem, s); break;
+    case 4: launch_ev<1, 1>(a, alch, energy, combine, grid, sms, resident, shmem, s); break;
+    case 5: launch_ev<1, 2>(a, alch, energy, combine, grid, sms, resident, shmem, s); break;
+    case 6: launch_ev<2, 0>(a, alch, energy, combine, grid, sms, resident, shmem, s); break;
+    case 7: launch_ev<2, 1>(a, alch, energy, combine, grid, sms, resident, shmem, s); break;
+    case 8: launch_ev<2, 2>(a, alch, energy, combine, grid, sms, resident, shmem, s); break;
     default: return BNB_ERR_ARG;
   }
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;

@@ -5,9 +5,11 @@
 #include "bnb_internal.h"
 
 namespace bnb {
-// alch: 0 none, 1 MSLD scaling, 2 MSLD + soft core.
+// alch: 0 none, 1 MSLD scaling, 2 MSLD + soft core.  grid: most CTAs; sms: SMs of
+// the device; resident: CTAs an SM holds, kept by the handle for one topology and
+// value of `energy` (0: asked for in this call).
 int launch_pair(const Dev &d, const PairConst &pc, const float *lambda, int elec, int vdw,
-                int alch, bool energy, bool count, int grid, cudaStream_t s);
+                int alch, bool energy, bool count, int grid, int sms, int &resident, cudaStream_t s);
 void launch_finalize(const Dev &d, const bnb_outputs &o, int mode, cudaStream_t s);
 // Sorts the work items by the cycles the last pair launch measured for them,
 // longest first, into Dev::order, which the following launches follow until
