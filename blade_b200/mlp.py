@@ -52,7 +52,7 @@ class BF16MLP:
                 lst.append(src[o:o + n])
             oW += pad(N * K)
             ob += pad(N)
-        self._views = [list(x) for x in (self.W, self.Wb, self.b, self.gW, self.gb, self.mW, self.mb, self.vW, self.vb)]
+        self._placed = self._layout()
         self._sync_bf16()
         M = max_batch
         self.xb = torch.empty(M * self.sizes[0], dtype=bf, device=self.dev)
@@ -69,11 +69,16 @@ class BF16MLP:
     def _s(self):
         return C.c_void_p(self.torch.cuda.current_stream().cuda_stream)
 
+    def _layout(self):
+        """Addresses and sizes of all tensors."""
+        t = [*self.W, *self.Wb, *self.b, *self.gW, *self.gb, *self.mW, *self.mb, *self.vW, *self.vb]
+        return list(map(self.torch.Tensor.data_ptr, t)), list(map(self.torch.Tensor.numel, t))
+
     def _whole(self):
-        """True while the lists hold the views made by __init__ (a caller may
-        put tensors of its own in them, such as clipped gradients)."""
-        lists = (self.W, self.Wb, self.b, self.gW, self.gb, self.mW, self.mb, self.vW, self.vb)
-        return all(a is b for x, y in zip(lists, self._views) for a, b in zip(x, y))
+        """True while every tensor lies where __init__ put it in the whole
+        buffers.  A caller may put tensors of its own in the lists, such as
+        clipped gradients, or give one other storage through its ``.data``."""
+        return self._layout() == self._placed
 
     def _sync_bf16(self):
         if self._whole():
@@ -142,8 +147,8 @@ class BF16MLP:
         parts = [(0, self._p.numel(), 0.0)] if weight_decay == 0.0 else \
             [(0, self._nW, weight_decay), (self._nW, self._p.numel(), 0.0)]
         for a, b, wd in parts:
-            _lib.call("bnb_mlp_adam", b - a, _p(self._p[a:b]), _p(self._pb[a:b]), _p(self._g[a:b]), _p(self._m[a:b]),
-                      _p(self._v[a:b]), lr, beta1, beta2, eps, wd, self.step_count, s)
+            at = [C.c_void_p(t.data_ptr() + a * t.element_size()) for t in (self._p, self._pb, self._g, self._m, self._v)]
+            _lib.call("bnb_mlp_adam", b - a, *at, lr, beta1, beta2, eps, wd, self.step_count, s)
 
     def train_step(self, x, target, weight=None, lr=1e-3, elem_weight=None):
         loss = self.loss_grad(x, target, weight, elem_weight)
