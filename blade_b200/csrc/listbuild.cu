@@ -652,16 +652,14 @@ __global__ void __launch_bounds__(kCullThreads) k_cull(Dev d, float rcull, float
   }
   int tiles[kWorkLevels], items[kWorkLevels];
   const int L = work_split(sTotal, ri.tilesPerWork, ri.tailTiles, tiles, items);
-  int s = sBase[0], done = 0;  // first candidate of the level, tail items before it
   for (int l = 0; l < L; l++) {
-    const int size = work_item_size(ri.tilesPerWork, l), end = s + tiles[l];
-    int2 *out = l == 0 ? d.work + sBase[2] : d.work + d.capWork + sBase[3] + done;
-    for (int k = threadIdx.x; k < items[l]; k += kCullThreads) {
-      const int first = s + k * size, n = end - first < size ? end - first : size;
+    const WorkLevel lv = work_level(sBase[0], ri.tilesPerWork, l, tiles, items);
+    int2 *out = (l == 0 ? d.work + sBase[2] : d.work + d.capWork + sBase[3]) + lv.before;
+    for (int k = threadIdx.x; k < lv.items; k += kCullThreads) {
+      int first, n;
+      lv.item(k, &first, &n);
       out[k] = make_int2(iBlock | (n << 22), first);
     }
-    if (l > 0) done += items[l];
-    s = end;
   }
 }
 

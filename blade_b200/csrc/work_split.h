@@ -41,19 +41,27 @@ BNB_HD inline int work_item_size(int T, int level) {
   return level == 0 ? T : ((T >> level) > 1 ? (T >> level) : 1);
 }
 
-// Walks the work items of one i block whose candidates are c0 .. c0+nc-1:
-// emit(level, k, first, n) for the k-th item of each level, levels in order,
-// items covering the candidates once, in order.
-template <class Emit>
-BNB_HD inline void work_walk(int c0, int nc, int T, int tailTiles, Emit emit) {
-  int tiles[kWorkLevels], items[kWorkLevels];
-  const int L = work_split(nc, T, tailTiles, tiles, items);
-  int s = c0;
-  for (int l = 0; l < L; l++) {
-    const int size = work_item_size(T, l), end = s + tiles[l];
-    for (int q = s, k = 0; q < end; q += size, k++) emit(l, k, q, end - q < size ? end - q : size);
-    s = end;
+// Work items of one level of one i block: item k (0 <= k < items) holds
+// candidates first + k size .. and has place before + k among the block's items
+// of its part of the list (full-size items, or tail items).
+struct WorkLevel {
+  int first, tiles, size, items, before;
+  BNB_HD void item(int k, int *firstTile, int *n) const {
+    *firstTile = first + k * size;
+    const int left = first + tiles - *firstTile;
+    *n = left < size ? left : size;
   }
+};
+
+// Level `level` of the block whose candidates begin at c0; tiles and items from
+// work_split.  The levels together cover the candidates once, in order.
+BNB_HD inline WorkLevel work_level(int c0, int T, int level, const int *tiles, const int *items) {
+  WorkLevel w{c0, tiles[level], work_item_size(T, level), items[level], 0};
+  for (int l = 0; l < level; l++) {
+    w.first += tiles[l];
+    if (l > 0) w.before += items[l];  // level 0 is a part of its own
+  }
+  return w;
 }
 
 }  // namespace bnb

@@ -1,12 +1,11 @@
 // Host-side check of the pair kernel's work-list split (bnb::work_split and
-// bnb::work_walk, the functions the list rebuild runs on the device): for
+// bnb::work_level, the functions the list rebuild runs on the device): for
 // every candidate count, tile count per item and tail length, the items of a
 // block cover its candidates once and in order, level by level, with item
-// sizes that never grow from one level to the next, and the per-level counts
-// that the rebuild reserves match the items written.  Prints "ok" or the
-// first failing case.
+// sizes that never grow from one level to the next, and the items of either
+// part of the list (full size, tail) take the places that the rebuild reserves,
+// each once.  Prints "ok" or the first failing case.
 #include <cstdio>
-#include <vector>
 
 #include "work_split.h"
 
@@ -25,21 +24,27 @@ int main() {
           return 1;
         }
         const int c0 = 1000;
-        int next = c0, lastLevel = 0, lastSize = 1 << 30;
-        std::vector<int> count(bnb::kWorkLevels, 0);
+        int next = c0, lastSize = 1 << 30, place[2] = {0, 0};  // places of the full-size and the tail items
         bool bad = false;
-        bnb::work_walk(c0, nc, T, tail * T, [&](int l, int k, int first, int n) {
-          const int size = bnb::work_item_size(T, l);
-          if (first != next || n < 1 || n > size || l < lastLevel || k != count[l] || size > lastSize) bad = true;
-          next = first + n;
-          if (l != lastLevel) lastSize = bnb::work_item_size(T, lastLevel);
-          lastLevel = l;
-          count[l]++;
-        });
-        for (int l = 0; l < bnb::kWorkLevels; l++)
-          if (count[l] != items[l]) bad = true;
+        for (int l = 0; l < L; l++) {
+          const bnb::WorkLevel w = bnb::work_level(c0, T, l, tiles, items);
+          int &at = place[l > 0];
+          if (w.items != items[l] || w.size != bnb::work_item_size(T, l) || w.size > lastSize || w.before != at)
+            bad = true;
+          lastSize = w.size;
+          for (int k = 0; k < w.items; k++) {
+            int first, n;
+            w.item(k, &first, &n);
+            if (first != next || n < 1 || n > w.size) bad = true;
+            next = first + n;
+          }
+          at += w.items;
+        }
+        int tail = 0;
+        for (int l = 1; l < bnb::kWorkLevels; l++) tail += items[l];
+        if (place[0] != items[0] || place[1] != tail) bad = true;
         if (bad || next != c0 + nc) {
-          std::printf("walk T=%d tail=%d nc=%d\n", T, tail, nc);
+          std::printf("items T=%d tail=%d nc=%d\n", T, tail, nc);
           return 1;
         }
       }
