@@ -144,7 +144,7 @@ struct Dev {
   uint32_t *masks;         // [capMask*32] word of j atom l: bit i clear = excluded from i atom i
   int *candStart;          // [maxBlocks] first candidate of the block (blocks in any order)
   int *candNum;            // [maxBlocks] its candidates
-  int2 *work;              // [2*capWork] (iBlock | tiles << 22, candidate start); tail items from capWork on
+  int2 *work;              // [2*capWork] (work_pack, candidate start); tail items from capWork on
   unsigned int *itemCost;  // [2*capWork] by place in the sequence full-size items, tail items: clock cycles of each work item in the last pair launch
   int *order;              // [2*capWork] work items by decreasing measured cost
   // --- per-step buffers -----------------------------------------------------

@@ -323,6 +323,19 @@ bool store_boxes(bnb_handle *h, const float *boxes) {
   return changed;
 }
 
+// Blocks a list over these boxes may have.
+long long max_blocks(const bnb_handle *h, const float *boxes) {
+  long long mb = 0;
+  for (int r = 0; r < h->R; r++) {
+    float b[3], t[3];
+    int dx, dy;
+    box_of(h, boxes, r, b, t);
+    bnb_domain_div(h->atomCount[r], b, &dx, &dy);
+    mb += h->atomCount[r] / 32 + (long long)dx * dy + 1;
+  }
+  return mb;
+}
+
 // Column grid per replica from its box; returns true if the layout changed.
 bool layout_columns(bnb_handle *h, const float *boxes) {
   bool changed = false;
@@ -683,6 +696,7 @@ int bnb_rebuild(bnb_handle *h, const float *position, const float *boxes, void *
     for (int k = 0; k < 3; k++)  // single-image scheme needs rCut <= half of every brick edge
       if (!(b[k] >= 2 * h->p.rCut) || !std::isfinite(t[k])) return BNB_ERR_ARG;
   }
+  if (max_blocks(h, boxes) >= bnb::kMaxListBlocks) return BNB_ERR_TOO_LARGE;
   cudaStream_t s = (cudaStream_t)stream;
   const bool async = (flags & BNB_ASYNC) != 0;
   bool changed = layout_columns(h, boxes);

@@ -396,8 +396,8 @@ __device__ __forceinline__ uint32_t excl_row(const Dev &d, int iBlock, int jBloc
 //      candidates come out in the order of a scan over codes and j blocks.  Hits
 //      are kept in shared memory (a piece with more than kHits is visited again).
 //    * One atomic each reserves the block's candidates, masks and work items, and
-//      the CTA writes them.  Work items: (iBlock | tiles << 22, first candidate),
-//      by work_split; the full-size ones from the start of the list, the tail
+//      the CTA writes them.  Work items: (block and tiles, first candidate), by
+//      work_split; the full-size ones from the start of the list, the tail
 //      after them (the pair kernel takes items in list order until it has
 //      measured them).
 //    Bound by the latencies one CTA sees in a row, so by CTAs in flight.  It
@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(kCullThreads) k_cull(Dev d, float rcull, float
     for (int k = threadIdx.x; k < lv.items; k += kCullThreads) {
       int first, n;
       lv.item(k, &first, &n);
-      out[k] = make_int2(iBlock | (n << 22), first);
+      out[k] = make_int2(work_pack(iBlock, n), first);
     }
   }
 }

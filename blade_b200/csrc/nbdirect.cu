@@ -729,8 +729,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairCtas) k_pair(KArgs A) {
     const int item = ordered ? d.order[w] : w;
     const long long tItem = clock64();
     const int2 wk = d.work[item < nFull ? item : d.capWork + item - nFull];
-    const int iBlock = wk.x & 0x3FFFFF;
-    const int c0 = wk.y, c1 = c0 + (wk.x >> 22);
+    const int iBlock = work_block(wk.x);
+    const int c0 = wk.y, c1 = c0 + work_tiles(wk.x);
     const RepInfo &ri = d.rep[d.blockRep[iBlock]];
     const float4 *shifts = ri.shift;  // image shift vectors by shift code
     const float4 imin = d.bmin[iBlock], imax = d.bmax[iBlock];
@@ -1158,7 +1158,6 @@ void launch_allpairs_ev(const AllPairsArgs &a, bool energy, dim3 grid, cudaStrea
 
 int launch_pair(const Dev &d, const PairConst &pc, const float *lambda, int elec, int vdw,
                 int alch, bool energy, bool count, int grid, int sms, int &resident, cudaStream_t s) {
-  if (32LL * d.maxBlocks >= (1LL << 27)) return BNB_ERR_TOO_LARGE;  // streamed entries hold the slot in 27 bits
   KArgs a{d, pc, lambda, count ? 1 : 0};
   size_t shmem = d.ljCombine ? 0 : sizeof(float2) * d.nTypes * d.nTypes;
   shmem = (shmem + 15) & ~size_t(15);

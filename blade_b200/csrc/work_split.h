@@ -13,6 +13,13 @@ namespace bnb {
 
 constexpr int kWorkLevels = 8;  // levels of the work list: items of T, T/2, ..., 1 tiles (T <= 32)
 
+// A work item holds its i block and tile count (1..32) in one word.  The rebuild
+// refuses lists of kMaxListBlocks blocks and more.
+constexpr int kWorkBlockBits = 22, kMaxListBlocks = 1 << kWorkBlockBits;
+BNB_HD inline int work_pack(int iBlock, int tiles) { return iBlock | (tiles << kWorkBlockBits); }
+BNB_HD inline int work_block(int packed) { return packed & (kMaxListBlocks - 1); }
+BNB_HD inline int work_tiles(int packed) { return packed >> kWorkBlockBits; }
+
 // Split of one i block's nc candidate tiles into work items.  Level 0 takes
 // the first nc - K tiles (K = min(nc, tailTiles)) in items of T tiles; the
 // last K tiles form the tail, which levels 1, 2, ... take from the front in

@@ -126,6 +126,9 @@ int bnb_set_box_type(bnb_handle *h, int triclinic);
  * cull loop, src/domdec/cull.cu:337-375); BNB_ASYNC = enqueue only (graph
  * capturable), overflow is reported through bnb_status and the pair kernel
  * then does no work.
+ * Limit: sum over the replicas of atoms / 32 + columns + 1 below 2^22 (134
+ * million atoms); above it the call returns BNB_ERR_TOO_LARGE and changes
+ * nothing.
  */
 #define BNB_ASYNC 1
 int bnb_rebuild(bnb_handle *h, const float *position, const float *boxes,

@@ -220,3 +220,21 @@ def test_pair_erfc_path_against_fp64(cuda):
         nb.close()
     assert worst_e <= 2e-6, worst_e
     assert worst_f <= 2e-6, worst_f
+
+
+def test_lists_beyond_the_block_index_are_refused(cuda):
+    """A work item holds its block in 22 bits: a cell with more columns than
+    that is refused before anything is allocated, and the handle goes on."""
+    s = systems.water_box()
+    nb = NbDirect(s)
+    pos = nb.positions_tensor()
+    nb.update_domdec(pos, True)
+    f = nb.evaluate(pos)[0]
+    free = torch.cuda.mem_get_info()[0]
+    with pytest.raises(_lib.BnbError) as e:
+        nb.update_domdec(pos, True, boxes=np.float32([1e11, 1e11, 24.0]))
+    assert e.value.code == 7 and torch.cuda.mem_get_info()[0] == free
+    assert torch.equal(f, nb.evaluate(pos)[0])           # the list built before still stands
+    nb.update_domdec(pos, True)
+    assert torch.equal(f, nb.evaluate(pos)[0])
+    nb.close()

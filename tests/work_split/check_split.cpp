@@ -6,10 +6,18 @@
 // part of the list (full size, tail) take the places that the rebuild reserves,
 // each once.  Prints "ok" or the first failing case.
 #include <cstdio>
+#include <initializer_list>
 
 #include "work_split.h"
 
 int main() {
+  // a work item's word: every tile count beside the first and the last block
+  for (int n = 1; n <= 32; n++)
+    for (int b : {0, 1, bnb::kMaxListBlocks - 1})
+      if (bnb::work_block(bnb::work_pack(b, n)) != b || bnb::work_tiles(bnb::work_pack(b, n)) != n) {
+        std::printf("pack block=%d tiles=%d\n", b, n);
+        return 1;
+      }
   const int tails[] = {0, 1, 2, 4, 8};
   for (int T = 1; T <= 32; T++)
     for (int tail : tails)
