@@ -376,12 +376,18 @@ double tiles_estimate(const bnb_handle *h, int r) {
 // (148 SMs x 16) an item each, by the estimate above, so that a small system is
 // spread over the GPU and a large one pays each item's set-up and half-empty
 // last round less often.  The estimate exceeds the real count by 1.1 (648
-// atoms, 9 A) to 1.5 times (3,000, 12 A), hence the factor.  It depends on the replica
-// alone, so a replica gives the same bits alone and in a batch.  Pair kernel,
+// atoms, 9 A) to 1.5 times (3,000, 12 A), hence the factor.  Pair kernel,
 // us, at 1 / 2 / 4 / 8 tiles an item: 648 atoms 15 / 16 / 20 / 28, 519 with
 // MSLD 19 / 25 / 34 / 56, 3,000 (12 A) 21 / 21 / 28 / 40, 20,577 (9 A)
-// 58 / 46 / 39 / 38, 23,558 (12 A) 105 / 82 / 70 / 66, 32 MSLD boxes of 690
-// atoms in a batch 100 / 80 / 68 / 75.
+// 58 / 46 / 39 / 38, 23,558 (12 A) 105 / 82 / 70 / 66.
+// Two sides of it cost time, and both are taken:
+//  * It depends on the replica alone, so that a replica gives the same bits alone
+//    and in a batch.  A batch of small replicas, which fills the GPU, would be
+//    faster with larger items: 32 MSLD boxes of 690 atoms 100 / 80 / 68 / 75, an
+//    evaluation of 100 water boxes of 648 atoms 144 at 2, 116 at 4, 102 at 8.  The
+//    caller's tuning is for them.
+//  * One tile is not taken for the smallest, although the 519-atom MSLD box would
+//    gain by it: batches of such boxes would lose more.
 int replica_tiles(const bnb_handle *h, int r) {
   const double items = tiles_estimate(h, r) / 1.5;
   int t = bnb::kMinAutoTiles;
@@ -865,10 +871,10 @@ int bnb_set_tuning(bnb_handle *h, int tilesPerWork, int ctasPerSM, int tailItems
   if (!h || tilesPerWork < bnb::kMinTilesPerWork || tilesPerWork > 32 || ctasPerSM < 0 || ctasPerSM > 8 ||
       tailItems < 0 || tailItems > 8)
     return BNB_ERR_ARG;
-  // the work items must be rebuilt; a first call that names the general default
-  // or the choice in effect leaves a built list valid
-  int t0, l0;
-  bnb_get_tuning(h, &t0, nullptr, &l0);
+  // The work items must be rebuilt.  A first call that names the general default
+  // or the choice in effect leaves a built list valid, with the items it has.
+  int t0 = h->tilesPerWork, l0 = h->tailItems;
+  if (!h->tuned) bnb_get_tuning(h, &t0, nullptr, &l0);
   const bool general = !h->tuned && tilesPerWork == bnb::kTilesPerWork && tailItems == bnb::kTailItems;
   if (!general && (tilesPerWork != t0 || tailItems != l0)) h->listBuilt = false;
   h->tuned = true;
@@ -878,17 +884,22 @@ int bnb_set_tuning(bnb_handle *h, int tilesPerWork, int ctasPerSM, int tailItems
   return BNB_OK;
 }
 
+// The split of the list in use (of the replica with the largest items), or
+// without one that of the next.
 int bnb_get_tuning(bnb_handle *h, int *tilesPerWork, int *ctasPerSM, int *tailItems) {
   if (!h) return BNB_ERR_ARG;
-  if (tilesPerWork) {
-    *tilesPerWork = h->tilesPerWork;
-    if (!h->tuned && h->listArena) {  // the largest of the replicas' own
-      *tilesPerWork = 0;
-      for (const RepInfo &ri : h->rep) *tilesPerWork = std::max(*tilesPerWork, ri.tilesPerWork);
-    }
+  int tiles = h->tilesPerWork, tail = h->tailItems;
+  if (h->listBuilt || (!h->tuned && h->listArena)) {
+    tiles = tail = 0;
+    for (const RepInfo &ri : h->rep)
+      if (ri.tilesPerWork > tiles) {
+        tiles = ri.tilesPerWork;
+        tail = ri.tailTiles / ri.tilesPerWork;
+      }
   }
+  if (tilesPerWork) *tilesPerWork = tiles;
   if (ctasPerSM) *ctasPerSM = h->ctasPerSM;
-  if (tailItems) *tailItems = h->tailItems;
+  if (tailItems) *tailItems = tail;
   return BNB_OK;
 }
 

@@ -391,10 +391,17 @@ int bnb_bias_f32(int blockCount, const float *lambda, const float *fixedBias,
  * i block become items of a quarter of the size, taken after all others, so
  * that the persistent warps finish close together (0 = no tail).  Until the
  * first call the library chooses the tiles per item of each replica from its
- * size (2, 4 or 8, no tail), and bnb_get_tuning reports those of the largest.
- * A changed tile count or tail takes effect at the next bnb_rebuild.  The
- * split of each block's tiles depends on its replica alone, so a replica gives
- * the same bits alone and in a batch at equal settings.  No reference
+ * size (2, 4 or 8, no tail).  The split of each block's tiles depends on its
+ * replica alone, so a replica gives the same bits alone and in a batch at equal
+ * settings (and in equal LJ modes: bnb_set_topology).  The price is paid by
+ * batches of many small replicas, which would fill the GPU with larger items: a
+ * batch of 100 boxes of 648 atoms takes 144 us an evaluation at their 2 tiles,
+ * 116 at 4 and 102 at 8 without tail; set or autotune the knobs there.
+ * A changed tile count or tail takes effect at the next bnb_rebuild, and a list
+ * built before it is no longer valid, except that a first call naming 8 tiles
+ * and tail 2, or the split in use, leaves the list valid as it is.
+ * bnb_get_tuning reports the split of the list in use (of its replica with the
+ * largest items), or of the next list while there is none.  No reference
  * counterpart.
  */
 int bnb_set_tuning(bnb_handle *h, int tilesPerWork, int ctasPerSM, int tailItems);

@@ -131,3 +131,33 @@ def test_water_beside_msld_replica_keeps_its_bits(cuda, n_side, methods):
         assert torch.equal(l[nb.lam_starts[r]:nb.lam_starts[r + 1]], m)
         one.close()
     nb.close()
+
+
+def test_tuning_reports_the_list_in_use(cuda):
+    """Naming the general default after a default build keeps that list, and its
+    split is the one reported; the next build has the bits of a handle tuned
+    before its first."""
+    s = systems.water_box(5)
+    nb = NbDirect(s)
+    pos = nb.positions_tensor()
+    nb.update_domdec(pos, True)
+    work = nb.list_sizes()["work"]
+    nb.set_tuning(8, 2)
+    assert nb.tuning() == {"tiles_per_work": 2, "ctas_per_sm": 2, "tail_items": 0}
+    nb.evaluate(pos)
+    assert nb.list_sizes()["work"] == work
+    nb.set_tuning(8, 2)                                   # once more: nothing changes
+    nb.evaluate(pos)
+    nb.update_domdec(pos, True)
+    assert nb.tuning() == {"tiles_per_work": 8, "ctas_per_sm": 2, "tail_items": 2}
+    one = NbDirect(s)
+    one.set_tuning(8)
+    assert one.tuning() == {"tiles_per_work": 8, "ctas_per_sm": 0, "tail_items": 2}
+    one.update_domdec(pos, True)
+    assert torch.equal(nb.evaluate(pos)[0], one.evaluate(pos)[0])
+    nb.set_tuning(4, 2)                                   # any other change asks for a rebuild
+    assert nb.tuning()["tiles_per_work"] == 4
+    with pytest.raises(Exception):
+        nb.evaluate(pos)
+    nb.close()
+    one.close()
