@@ -1370,8 +1370,14 @@ extern "C" int bnb_set_pme(bnb_handle *h, int order, float gridSpace, const int 
   free_pme(h);
   // Own transforms for all replicas or cuFFT for all.  A plane (one x) of a grid
   // is transformed by one CTA in shared memory, which ends at about 165^2
-  // points, and the radices are 2 to 8.  Faster than cuFFT at every size it
-  // takes (pmefft.cu).
+  // points, and the radices are 2 to 8.  One evaluation with 1,536 atoms a
+  // replica, own / cuFFT, us: 64^3 30 / 51, 8 of them 67 / 86; 96^3 41 / 58, 8 of
+  // them 164 / 210; 100^3 45 / 56, 8 of them 191 / 181; 128^3 59 / 66, 8 of them
+  // 397 / 307; 144^3 74 / 78; 160^3 119 / 108; 600 x 64 x 64 62 / 83.  cuFFT is
+  // faster where planes that fill half an SM's shared memory or more come in more
+  // than one wave.  The own transforms are kept there too: a rule on the number of
+  // planes would give a replica other bits in a batch than alone, for 90 of 1,038
+  // us with 8 replicas of 192,000 atoms on 128^3.
   bool own = true;
   bnb::PmeFftLaunch fl{};
   std::vector<float2> twiddle;
@@ -1384,6 +1390,7 @@ extern "C" int bnb_set_pme(bnb_handle *h, int order, float gridSpace, const int 
     const size_t ps = bnb::pme_fft_plane_smem(K, &be), xs = bnb::pme_fft_x_smem(K[0]);
     own = own && ps <= bnb::kPmeFftSmem && xs <= bnb::kPmeFftSmem;
     fl.xSmem = std::max(fl.xSmem, xs);
+    fl.xThreads = std::max(fl.xThreads, std::min(512, 128 * ((K[0] + 159) / 160)));
     bufElems = std::max(bufElems, be);
     maxPlane = std::max(maxPlane, K[1] * K[2]);
   }
@@ -1405,13 +1412,21 @@ extern "C" int bnb_set_pme(bnb_handle *h, int order, float gridSpace, const int 
     fl.planes = (int)planeMap.size();
     fl.colTiles = (int)colMap.size();
     fl.planeSmem = sizeof(float2) * (2 * (size_t)bufElems + tables);
-    // one CTA per SM at most: about 4 points a thread, the passes are latency in
-    // a row (64^3: 52 -> 47 us an evaluation against 16 points); more planes
-    // than SMs: 16, so that CTAs share an SM (8 replicas of 36^3 to 54^3: a step
-    // 370 -> 359 us against 4)
-    const int points = fl.planes <= 148 ? 4 : 16;
-    fl.planeThreads = 128;
-    while (fl.planeThreads < 1024 && points * fl.planeThreads < maxPlane) fl.planeThreads *= 2;
+    // One CTA per SM at most: about 4 points a thread, the passes are latency in
+    // a row (64^3: 52 -> 47 us an evaluation against 16 points).  More planes than
+    // SMs: 8 points, and no more threads than lets an SM hold the CTAs that its
+    // shared memory holds (40 registers a thread, 1,536 threads); with 1,024 an SM
+    // had one CTA at a time: 8 of 96^3 207 -> 164, 8 of 100^3 228 -> 191, 160 x
+    // 100 x 100 68 -> 60.
+    const int sms = 148, wave = (fl.planes + sms - 1) / sms;
+    const int fit = (int)(228 * 1024 / (fl.planeSmem + 1024)), ctas = std::max(1, std::min(fit, wave));
+    if (wave <= 1) {
+      fl.planeThreads = 128;
+      while (fl.planeThreads < 1024 && 4 * fl.planeThreads < maxPlane) fl.planeThreads *= 2;
+    } else {
+      const int want = (maxPlane / 8 + 31) / 32 * 32, most = 1536 / ctas / 32 * 32;
+      fl.planeThreads = std::max(128, std::min(std::min(want, most), 1024));
+    }
     own = fl.planeSmem <= bnb::kPmeFftSmem && bnb::pme_fft_setup() == BNB_OK;
   }
   if (!own) {

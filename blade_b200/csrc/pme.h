@@ -48,7 +48,7 @@ struct PmeArgs {
 };
 
 struct PmeFftLaunch {
-  int planes, planeThreads, colTiles;
+  int planes, planeThreads, colTiles, xThreads;
   size_t planeSmem, xSmem;
 };
 

@@ -15,7 +15,8 @@
 // traffic: 64^3 takes 2 passes per direction, 128^3 three.  Measured against the
 // cuFFT path (conversion, three kernels each way, convolution), one evaluation
 // at order 6: 20^3 41 -> 25 us, 64^3 57 -> 47, 128^3 207 -> 196, and a step of 8
-// replicas with six grid sizes 437 -> 359 us.
+// replicas with six grid sizes 437 -> 359 us; where cuFFT is the faster is said at
+// the choice in bnb_set_pme.
 #include <cuda_runtime.h>
 
 #include "pme.h"
@@ -240,8 +241,11 @@ __global__ void __launch_bounds__(1024) k_pme_plane_inverse(PmeArgs a) {
   }
 }
 
-// Tile of kPmeCols neighbouring columns (64 bytes of every x plane).
-__global__ void __launch_bounds__(128) k_pme_x(PmeArgs a) {
+// Tile of kPmeCols neighbouring columns (64 bytes of every x plane).  128 threads
+// for each 160 points along x: with 128 in all, long grids had few warps to hide
+// the passes' latency (an evaluation on 300 x 64 x 64 57 -> 47 us, on 600 x 64 x 64
+// 84 -> 62).
+__global__ void __launch_bounds__(512, 2) k_pme_x(PmeArgs a) {
   pdl_wait();
   extern __shared__ __align__(16) float2 fsm[];
   const int2 at = a.colMap[blockIdx.x];  // (replica, first column)
@@ -321,7 +325,7 @@ int pme_fft_setup() {
 
 int pme_fft(const PmeArgs &a, const PmeFftLaunch &l, cudaStream_t s) {
   launch_pdl(k_pme_plane_forward, l.planes, l.planeThreads, l.planeSmem, s, a);
-  launch_pdl(k_pme_x, l.colTiles, 128, l.xSmem, s, a);
+  launch_pdl(k_pme_x, l.colTiles, l.xThreads, l.xSmem, s, a);
   launch_pdl(k_pme_plane_inverse, l.planes, l.planeThreads, l.planeSmem, s, a);
   return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }

@@ -78,3 +78,28 @@ def test_sizes_of_the_spread_and_gather(cuda, order, side, box):
     # FP32 grid values: relative to the scale of the largest terms, which cancel in few waters
     assert np.sqrt(((f - go) ** 2).sum()) <= 2e-5 * max(np.sqrt((go ** 2).sum()), 1e-2)
     assert abs(e[0] - eo) <= 2e-5 * max(abs(eo), s.N)
+
+
+@pytest.mark.parametrize("grids", [[(96, 96, 96), (80, 100, 96)], [(162, 30, 32), (32, 30, 18)], [(162, 100, 100)],
+                                   [(48, 48, 48)] * 3 + [(640, 16, 16)]])
+def test_launch_shapes_keep_the_bits(cuda, grids):
+    """More planes than SMs and long edges change the threads of a CTA (fewer a
+    plane, more a tile of columns), not the results."""
+    reps = [systems.msld_water(30 + k % 2) for k in range(len(grids))]
+    nb = NbDirect(reps)
+    nb.set_pme(6, grid=grids)
+    f, l, e = _run(nb)
+    lam = nb.lambdas_tensor().cpu().numpy().astype(np.float64)
+    for r, s in enumerate(reps):
+        one = NbDirect(s)
+        one.set_pme(6, grid=[grids[r]])
+        f1, l1, e1 = _run(one)
+        one.close()
+        at = slice(nb.starts[r], nb.starts[r + 1])
+        assert np.array_equal(f[at], f1) and e[r] == e1[0]
+        eo, go, _, _ = pme_oracle.pme_recip(s.xyz, s.nbonds["q"], s.box, grids[r], 6, float(np.float32(s.betaEwald)),
+                                            float(np.float32(systems.KELEC_AKMA)), s.nbonds["siteBlock"],
+                                            lam[nb.lam_starts[r]:nb.lam_starts[r + 1]])
+        assert np.sqrt(((f[at] - go) ** 2).sum()) <= 1e-5 * np.sqrt((go ** 2).sum())
+        assert abs(e[r] - eo) <= 1e-5 * abs(eo)
+    nb.close()
