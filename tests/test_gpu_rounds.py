@@ -161,3 +161,26 @@ def test_tuning_reports_the_list_in_use(cuda):
         nb.evaluate(pos)
     nb.close()
     one.close()
+
+
+@pytest.mark.parametrize("r", [0.12, 0.2, 0.4])
+@pytest.mark.parametrize("pick", [(1, 302), (2, 500)])
+def test_pair_energies_beyond_the_fast_range(cuda, pick, r):
+    """Hydrogens of two molecules close enough for pair energies of some hundreds
+    to 4e5: with the ordinary ones they share a step, whose sum switches to the
+    general conversion at 1000."""
+    s = systems.water_box(8)
+    x = s.xyz.copy()
+    i, j = pick
+    mol = 3 * (j // 3)
+    x[mol:mol + 3] += x[i] + np.float32([r, 0, 0]) - x[j]  # the whole molecule of j beside i
+    s.xyz = x
+    nb = NbDirect(s)
+    pos = nb.positions_tensor()
+    nb.update_domdec(pos, True)
+    _, _, e = nb.evaluate(pos)
+    o = oracle.nbdirect(s)
+    assert nb.status() == 0
+    # FP32 coordinates decide the distance: the oracle sees the same ones
+    assert abs(float(e[0]) - o["energy"]) <= TOL * max(abs(o["energy"]), s.N)
+    nb.close()
