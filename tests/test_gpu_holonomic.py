@@ -82,17 +82,18 @@ def test_split_step_equals_fused(cuda):
     outs = []
     for split in (False, True):
         x, v, th, vt = _t(x0), _t(v0), _t(t0), _t(vt0)
+        f, m, ft, mt = _t(f0), _t(ism), _t(ft0), _t(ismt)  # held: a freed one would give its memory to the next
         xf = torch.zeros(nx, dtype=torch.float32, device="cuda")
         args = (P(x), P(v))
         if split:
             xp = torch.zeros(nx, dtype=torch.float64, device="cuda")
             for phase in (0, 1):
-                _lib.call("bnb_langevin_half", phase, nx, nt, P(x), P(v), P(xp), P(_t(f0)), P(_t(ism)), P(th), P(vt),
-                          P(_t(ft0)), P(_t(ismt)), 0.04, 0.9, 0.3, 0.95, 0.2, C.c_ulonglong(11), C.c_ulonglong(5),
+                _lib.call("bnb_langevin_half", phase, nx, nt, P(x), P(v), P(xp), P(f), P(m), P(th), P(vt),
+                          P(ft), P(mt), 0.04, 0.9, 0.3, 0.95, 0.2, C.c_ulonglong(11), C.c_ulonglong(5),
                           None, P(xf), None, None)
         else:
-            _lib.call("bnb_langevin_vrorv", nx, nt, *args, P(_t(f0)), P(_t(ism)), P(th), P(vt), P(_t(ft0)),
-                      P(_t(ismt)), 0.04, 0.9, 0.3, 0.95, 0.2, C.c_ulonglong(11), C.c_ulonglong(5), None, P(xf),
+            _lib.call("bnb_langevin_vrorv", nx, nt, *args, P(f), P(m), P(th), P(vt), P(ft),
+                      P(mt), 0.04, 0.9, 0.3, 0.95, 0.2, C.c_ulonglong(11), C.c_ulonglong(5), None, P(xf),
                       None, None)
         torch.cuda.synchronize()
         outs.append((x.cpu(), v.cpu(), th.cpu(), vt.cpu(), xf.cpu()))
