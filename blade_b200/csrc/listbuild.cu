@@ -467,8 +467,12 @@ __global__ void __launch_bounds__(kCullThreads) k_cull(Dev d, float rcull, float
       y0 = max(y0, (int)floorf((imin.y - rcull - sv.y) * by) - 1);
       y1 = min(y1, (int)floorf((imax.y + rcull - sv.y) * by) + 1);
     }
-    ny = y1 - y0 + 1;
-    cells = x1 < x0 || ny <= 0 ? 0 : (x1 - x0 + 1) * ny;
+    // the box of a block that has no finite x or y is (inf, -inf): its range ends at
+    // the limits of int, where a difference would wrap
+    if (x0 <= x1 && y0 <= y1) {
+      ny = y1 - y0 + 1;
+      cells = (x1 - x0 + 1) * ny;
+    }
   }
   int all = cells;
 #pragma unroll

@@ -238,3 +238,32 @@ def test_lists_beyond_the_block_index_are_refused(cuda):
     nb.update_domdec(pos, True)
     assert torch.equal(f, nb.evaluate(pos)[0])
     nb.close()
+
+
+@pytest.mark.parametrize("axes", [(0,), (1,), (2,), (0, 1), (0, 1, 2)])
+@pytest.mark.parametrize("n", [20, 33, 648])
+def test_blocks_without_a_finite_coordinate(cuda, n, axes):
+    """Blocks whose atoms are all NaN in some axes, whole ones and ones with empty
+    slots (whose box is (inf, -inf) there): flagged, and the handle goes on."""
+    s = systems.water_box()
+    s = dataclasses.replace(s, xyz=s.xyz[:n].copy(), nbonds=s.nbonds[:n].copy(), excl=s.excl[(s.excl < n).all(1)])
+    nb = NbDirect(s)
+    pos = nb.positions_tensor()
+    nb.update_domdec(pos, True)
+    ref = nb.get_list()
+    bad = pos.clone()
+    for k in axes:
+        bad[k::3] = float("nan")
+    nb.update_domdec(bad, True)
+    nb.evaluate(bad)
+    assert nb.status(clear=True) & _lib.STATUS_NONFINITE
+    half = pos.clone()                                    # some blocks only
+    half[axes[0]::6] = float("nan")
+    nb.update_domdec(half, True)
+    nb.evaluate(half)
+    assert nb.status(clear=True) & _lib.STATUS_NONFINITE
+    nb.update_domdec(pos, True)
+    assert nb.status() == 0
+    again = nb.get_list()
+    assert all(np.array_equal(ref[k], again[k]) for k in ref)
+    nb.close()
