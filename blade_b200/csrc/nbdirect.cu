@@ -815,7 +815,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairCtas) k_pair(KArgs A) {
       if (act) nxt.fetch(d, cand, __ffs(act) - 1, lane);
       const float4 sv = shifts[cur.code];
       const float4 xj = make_float4(cur.xj.x + sv.x, cur.xj.y + sv.y, cur.xj.z + sv.z, cur.xj.w);
-      uint32_t mask = cur.mask;
+      uint32_t mask = xj.x > 1.0e17f ? 0u : cur.mask;  // empty slots would pass the test against a box of NaN
       if (cur.jBlock == iBlock && cur.code == 0) mask &= (1u << lane) - 1u;  // each pair of the block once: i < j
 
       const bool toM = ALCH && (anyI || cur.siteBlock != 0);
@@ -863,7 +863,11 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairCtas) k_pair(KArgs A) {
     }
     // the groups hold the same i atoms: after the sum lane l has atom l
     const float fix = sum_groups(fx, lane), fiy = sum_groups(fy, lane), fiz = sum_groups(fz, lane);
-    if (fix != 0.f || fiy != 0.f || fiz != 0.f) {
+    // A NaN among the j atoms makes the sums of empty i slots NaN too, and nothing
+    // clears their accumulators; lane l holds atom l's position among its four.
+    const float2 xl = lane & 8 ? I.x[1] : I.x[0];
+    const bool empty = (lane & 16 ? xl.y : xl.x) < -1.0e17f;
+    if (!empty && (fix != 0.f || fiy != 0.f || fiz != 0.f)) {
       const int islot = 32 * iBlock + lane;
       red_add(&d.accF[islot], to_fix(fix));
       red_add(&d.accF[NS + islot], to_fix(fiy));

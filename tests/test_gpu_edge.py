@@ -250,7 +250,7 @@ def test_blocks_without_a_finite_coordinate(cuda, n, axes):
     nb = NbDirect(s)
     pos = nb.positions_tensor()
     nb.update_domdec(pos, True)
-    ref = nb.get_list()
+    ref, _, e_ref = nb.evaluate(pos)
     bad = pos.clone()
     for k in axes:
         bad[k::3] = float("nan")
@@ -263,7 +263,7 @@ def test_blocks_without_a_finite_coordinate(cuda, n, axes):
     nb.evaluate(half)
     assert nb.status(clear=True) & _lib.STATUS_NONFINITE
     nb.update_domdec(pos, True)
+    f, _, e = nb.evaluate(pos)
     assert nb.status() == 0
-    again = nb.get_list()
-    assert all(np.array_equal(ref[k], again[k]) for k in ref)
+    assert torch.equal(f, ref) and torch.equal(e, e_ref)
     nb.close()
