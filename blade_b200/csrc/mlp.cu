@@ -258,6 +258,16 @@ __global__ void __launch_bounds__(T == 64 ? 256 : 128) k_gemm_bf16(Products ps) 
   }
 }
 
+// Y, Yf = act(Z), where the product's own epilogue may not write them.
+__global__ void k_act(int n, const float *Z, int act, uint16_t *Y, float *Yf) {
+  pdl_wait();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const float z = Z[t], y = act ? z * sigmoid(z) : z;
+  if (Y) Y[t] = f2bf(y);
+  if (Yf) Yf[t] = y;
+}
+
 // dZ = dY act'(Z): FP32 copy, BF16 copy (for the products) and its column
 // sums db[n] = sum_m dZ[m,n].  A CTA owns 32 columns and takes 128 rows at a
 // time with all its threads; the sum of a column is 8 slices (slice r adds
@@ -390,6 +400,11 @@ __global__ void k_to_bf16(int n, const float *x, uint16_t *y) {
 }
 
 inline int grid1(long long n) { return (int)((n + 255) / 256); }
+// Whether a bytes from p and b bytes from q share memory (null: no).
+inline bool overlap(const void *p, size_t a, const void *q, size_t b) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(p), y = reinterpret_cast<uintptr_t>(q);
+  return x && y && x < y + b && y < x + a;
+}
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 inline bool aligned8(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; }
 
@@ -436,10 +451,19 @@ extern "C" int bnb_mlp_linear_forward(int M, int N, int K, const uint16_t *X, co
   if (M < 0 || N < 0 || K < 0 || !X || !W || !Z || (act != 0 && act != 1)) return BNB_ERR_ARG;
   if ((long long)M * N >= (1ll << 31)) return BNB_ERR_ARG;
   if (M == 0 || N == 0) return BNB_OK;
+  // A layer in place (Y over X): other tiles still read the inputs while one writes
+  // its outputs, so the activation is a launch of its own.
+  const size_t n = (size_t)M * N, k2 = 2 * (size_t)K;
+  const bool apart = !overlap(Y, 2 * n, X, M * k2) && !overlap(Yf, 4 * n, X, M * k2) && !overlap(Y, 2 * n, W, N * k2) &&
+                     !overlap(Yf, 4 * n, W, N * k2) && !overlap(Y, 2 * n, bias, 4 * (size_t)N) &&
+                     !overlap(Yf, 4 * n, bias, 4 * (size_t)N);
   Products ps{};
   // Z[m,n] = sum_k X[m,k] W[n,k]
-  ps.p[0] = Product{X, W, M, N, K, 0, 0, 0, 0, Z, bias, act, Y, Yf};
-  return gemm(ps, 1, (cudaStream_t)stream);
+  ps.p[0] = Product{X, W, M, N, K, 0, 0, 0, 0, Z, bias, act, apart ? Y : nullptr, apart ? Yf : nullptr};
+  const int rc = gemm(ps, 1, (cudaStream_t)stream);
+  if (rc || apart) return rc;
+  launch_pdl(k_act, grid1((long long)n), 256, 0, (cudaStream_t)stream, (int)n, Z, act, Y, Yf);
+  return cudaGetLastError() == cudaSuccess ? BNB_OK : BNB_ERR_CUDA;
 }
 
 extern "C" int bnb_mlp_linear_backward(int M, int N, int K, const float *dY, const float *Z, int act,
@@ -453,10 +477,15 @@ extern "C" int bnb_mlp_linear_backward(int M, int N, int K, const float *dY, con
   launch_pdl(k_act_grad, (N + 31) / 32, 1024, 0, s, M, N, dY, Z, act, dZ, dZb, db);
   if (cudaGetLastError() != cudaSuccess) return BNB_ERR_CUDA;
   if (K == 0) return BNB_OK;
-  Products ps{};
-  ps.p[0] = Product{dZb, X, N, K, M, 1, 1, 0, 0, dW, nullptr, 0, nullptr, nullptr};  // dW[n,k] = sum_m dZ[m,n] X[m,k]
-  ps.p[1] = Product{dZb, W, M, K, N, 0, 1, 0, 0, dX, nullptr, 0, nullptr, nullptr};  // dX[m,k] = sum_n dZ[m,n] W[n,k]
-  return gemm(ps, dX ? 2 : 1, s);
+  // dW[n,k] = sum_m dZ[m,n] X[m,k], dX[m,k] = sum_n dZ[m,n] W[n,k]
+  const Product w{dZb, X, N, K, M, 1, 1, 0, 0, dW, nullptr, 0, nullptr, nullptr};
+  const Product x{dZb, W, M, K, N, 0, 1, 0, 0, dX, nullptr, 0, nullptr, nullptr};
+  Products both{{w, x}};
+  if (!dX || !overlap(dX, 4 * (size_t)M * K, X, 2 * (size_t)M * K)) return gemm(both, dX ? 2 : 1, s);
+  // dX over X, which dW reads first
+  Products first{{w, w}}, second{{x, x}};
+  const int rc = gemm(first, 1, s);
+  return rc ? rc : gemm(second, 1, s);
 }
 
 extern "C" int bnb_mlp_mse(int M, int N, const float *Y, const float *T, const float *weight,

@@ -196,3 +196,50 @@ def test_adam_step_takes_the_callers_gradients(cuda):
     b.mW[0].zero_()
     b.adam_step()
     assert torch.equal(b.W[0], before)
+
+
+@pytest.mark.parametrize("n", [24, 50, 200])
+def test_layers_over_their_inputs(cuda, n):
+    """A layer may write its output over its input (or weights), and its input
+    gradient over its input: the results of separate buffers."""
+    M = 300
+    rng = np.random.default_rng(n)
+    x, w = rng.normal(size=(M, n)).astype(np.float32), (rng.normal(size=(n, n)) / np.sqrt(n)).astype(np.float32)
+    bias, dY = torch.randn(n, device="cuda"), torch.randn(M * n, device="cuda")
+
+    def buffers():
+        X, W = (torch.empty(a.size, dtype=torch.int16, device="cuda") for a in (x, w))
+        for a, d in ((x, X), (w, W)):
+            src = torch.as_tensor(a, device="cuda")
+            _lib.call("bnb_to_bf16", a.size, _p(src), _p(d), _s())
+            torch.cuda.synchronize()
+        return X, W, torch.empty(M * n, device="cuda")
+
+    def forward(X, W, Z, Y, Yf):
+        _lib.call("bnb_mlp_linear_forward", M, n, n, _p(X), _p(W), _p(bias), 1, _p(Z), _p(Y), _p(Yf), _s())
+
+    X, W, Z = buffers()
+    Y, Yf = torch.empty(M * n, dtype=torch.int16, device="cuda"), torch.empty(M * n, device="cuda")
+    forward(X, W, Z, Y, Yf)
+    X2, W2, Z2 = buffers()
+    forward(X2, W2, Z2, X2, None)                         # Y over X
+    assert torch.equal(Z, Z2) and torch.equal(Y, X2)
+    X3, W3, Z3 = buffers()
+    both = torch.empty(M * n, device="cuda")              # Yf over X, which lies in its second half
+    both.view(torch.int16)[M * n:].copy_(X3)
+    forward(both.view(torch.int16)[M * n:], W3, Z3, None, both)
+    assert torch.equal(Z, Z3) and torch.equal(Yf, both)
+
+    def backward(X, W, dX):
+        dZ, dZb = torch.empty(M * n, device="cuda"), torch.empty(M * n, dtype=torch.int16, device="cuda")
+        dW, db = torch.empty(n * n, device="cuda"), torch.empty(n, device="cuda")
+        _lib.call("bnb_mlp_linear_backward", M, n, n, _p(dY), _p(Z), 1, _p(X), _p(W), _p(dZ), _p(dZb), _p(dX), _p(dW),
+                  _p(db), _s())
+        return dW, db
+
+    dX = torch.empty(M * n, device="cuda")
+    dW, db = backward(X, W, dX)
+    over = torch.empty(M * n, device="cuda")
+    over.view(torch.int16)[:M * n].copy_(X)               # X in the first half of its gradient's memory
+    dW2, db2 = backward(over.view(torch.int16)[:M * n], W, over)
+    assert torch.equal(dW, dW2) and torch.equal(db, db2) and torch.equal(dX, over)
