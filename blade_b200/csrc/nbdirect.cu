@@ -246,8 +246,8 @@ __device__ __forceinline__ float general_pair(const PairConst &pc, float r2, flo
 
 // ---------------------------------------------------------------------------
 // Packed FP32x2 arithmetic (sm_100): one instruction updates the .x and .y
-// halves, which the streamed tile path below uses for two independent pairs
-// (A in .x, B in .y) of one lane.
+// halves, which the rounds below use for two independent pairs (A in .x, B in .y)
+// of one lane.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
@@ -686,9 +686,12 @@ struct WarpSmem<COMBINE, 0> {
   Queue<COMBINE, false, kPlainPlaces> plain;
 };
 
-// Resident warps, at 128 registers: 16 in 2 CTAs.  18 warps (3 x 6, 112
-// registers) and 20 (4 x 5, 96) spill: chain of 23,558 atoms 697 -> 724 and 738 us a
-// ten-step pass, 32 MSLD boxes 1025 -> 1113 and 1163; 4 CTAs of 4 the same as 2 of 8.
+// Resident warps, at 128 registers: 16 in 2 CTAs.  Most variants spill a little
+// there too (79 of 108; bytes stored / loaded, PME + VFSWITCH: force only 12 / 12 in
+// table and 32 / 24 in combination mode, soft core 36 to 96 / 32 to 64, with energy up to
+// 120 / 88).  18 warps (3 x 6, 112 registers) and 20 (4 x 5, 96) spill more: chain
+// of 23,558 atoms 697 -> 724 and 738 us a ten-step pass, 32 MSLD boxes 1025 -> 1113
+// and 1163; 4 CTAs of 4 the same as 2 of 8.
 constexpr int kPairWarps = 8, kPairCtas = 2;
 
 // ---------------------------------------------------------------------------
